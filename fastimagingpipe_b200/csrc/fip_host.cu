@@ -1281,8 +1281,7 @@ int fip_plane_project(const float* uvw, const float* freqs, size_t rows, size_t 
                       float* V, void* stream) {
   if (!uvw || !freqs || !B || !V) return fail(FIP_ERR_ARG, "null device pointer");
   if (rows == 0 || chans == 0) return fail(FIP_ERR_ARG, "empty measurement set");
-  FIP_CUDA(fip_launch_plane_project(uvw, freqs, rows, chans, nullptr, B, V,
-                                    (cudaStream_t)stream));
+  FIP_CUDA(fip_launch_plane_project(uvw, freqs, rows, chans, B, V, (cudaStream_t)stream));
   return FIP_OK;
 }
 

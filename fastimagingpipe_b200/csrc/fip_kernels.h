@@ -150,8 +150,7 @@ cudaError_t fip_launch_pixel_targets(const FipGeom& geo, const float* V, float* 
 
 // ---- plane projection (fip_precise.cu) ----
 cudaError_t fip_launch_plane_project(const float* uvw, const float* freqs, size_t rows,
-                                     size_t chans, double* work, float* B, float* V,
-                                     cudaStream_t s);
+                                     size_t chans, float* B, float* V, cudaStream_t s);
 cudaError_t fip_launch_collapse(const float* v0r, const float* v0i, const float* v3r,
                                 const float* v3i, const unsigned char* f0,
                                 const unsigned char* f3, const float* w0, const float* w3,
