@@ -97,6 +97,34 @@ struct FipGridSnap {
   int layout;               // grid layout (FipGeom::layout)
 };
 
+// One snapshot of a binning launch: its coordinates, grid geometry and bins
+// (FipBins).  base (or null): per-CTA list positions [ctas][ntiles]; grid (or
+// null): the grid whose split tiles the scatter pass zeroes.
+struct FipBinSnap {
+  const float* B;  // [nb][2]
+  int nb;
+  float scale;     // cell * G
+  int g, hp, tiles_c, ntiles, layout;
+  unsigned wcap;
+  unsigned* count;
+  unsigned* offset;
+  unsigned* cursor;
+  unsigned* base;
+  unsigned* entries;
+  int4* work;
+  unsigned* nwork;
+  unsigned* bbox;
+  unsigned* multi;
+  unsigned* nmulti;
+  float2* grid;
+};
+
+// The snapshots of one binning launch (a kernel parameter of about 8.2 KB).
+struct FipBinBatch {
+  int count;
+  FipBinSnap s[FIP_MAX_BATCH];
+};
+
 // The snapshots of one batched gridding launch (a kernel parameter of
 // about 5.6 KB).
 struct FipGridBatch {

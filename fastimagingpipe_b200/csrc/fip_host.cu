@@ -374,7 +374,7 @@ static void imager_free(fip_imager* im) {
   for (Lane& L : im->lane) {
     if (L.stream) cudaStreamSynchronize(L.stream);
     if (L.plan_ok) cufftDestroy(L.plan);
-    void* lp[] = {L.grid, L.bins.count, L.bins.offset, L.bins.cursor, L.bins.entries,
+    void* lp[] = {L.grid, L.bins.count, L.bins.offset, L.bins.cursor, L.bins.base, L.bins.entries,
                   L.bins.work, L.bins.nwork, L.bins.bbox, L.bins.multi, L.bins.nmulti,
                   L.colbuf, L.pre, L.targets, L.q_re, L.q_im, L.q_scale};
     for (void* p : lp)
@@ -541,6 +541,8 @@ int fip_imager_create(fip_imager** out, const fip_imager_config* cfg) {
     FIP_ALLOC(dalloc(&L.bins.count, ntiles, tot));
     FIP_ALLOC(dalloc(&L.bins.offset, ntiles + 1, tot));
     FIP_ALLOC(dalloc(&L.bins.cursor, ntiles, tot));
+    if (fip_bin_batchable(geo))
+      FIP_ALLOC(dalloc(&L.bins.base, (size_t)fip_bin_ctas(1, nb) * ntiles, tot));
     FIP_ALLOC(dalloc(&L.bins.entries, L.bins.cap, tot));
     FIP_ALLOC(dalloc(&L.bins.work, L.bins.wcap, tot));
     FIP_ALLOC(dalloc(&L.bins.nwork, 1, tot));
@@ -658,7 +660,7 @@ static int image_snapshot_impl(fip_imager* im, Lane& L, const float* vr, const f
     if (fork) FIP_CUDA(cudaEventRecord(im->ev_join, im->side));
   }
   k = stage_begin(im, ST_BIN, s);
-  FIP_CUDA(fip_launch_bin(geo, B, (int)nb, L.bins, s));
+  FIP_CUDA(fip_launch_bin(geo, B, (int)nb, L.bins, L.grid, s));
   stage_end(im, k, s);
   // The host path stages the visibilities while the binning runs: the
   // gridding (and the reduced-storage conversion) wait for them.
@@ -683,7 +685,7 @@ static int image_snapshot_impl(fip_imager* im, Lane& L, const float* vr, const f
   FIP_CUDA(fip_launch_grid(geo, B, gvr, gvi, vt, L.q_scale, V, (int)nb, L.bins, L.grid,
                            grid_compensated(precise, vt), s, im->grid_ctas_per_sm, raw));
   stage_end(im, k, s);
-  im->launches += fip_bin_launches(geo) + 2;  // binning, zero tiles, grid
+  im->launches += fip_bin_launches(geo) + 1;  // binning, grid
   if (im->custom_fft) {
     k = stage_begin(im, ST_FFT_COLS, s);
     FIP_CUDA(fip_launch_fft_cols(geo, L.grid, L.bins.bbox, L.colbuf, im->twiddles, im->fft, s));
@@ -847,12 +849,12 @@ int fip_grid_snapshot(fip_imager* im, const float* vis_re, const float* vis_im, 
     gvr = L.q_re;
     gvi = L.q_im;
   }
-  FIP_CUDA(fip_launch_bin(geo, B, (int)nb, L.bins, s));
+  FIP_CUDA(fip_launch_bin(geo, B, (int)nb, L.bins, reinterpret_cast<float2*>(grid), s));
   FIP_CUDA(fip_launch_grid(geo, B, gvr, gvi, vt, L.q_scale, V, (int)nb, L.bins,
                            reinterpret_cast<float2*>(grid), grid_compensated(precise, vt), s,
                            im->grid_ctas_per_sm));
   im->last_lane = 0;
-  im->launches += fip_bin_launches(geo) + 2;
+  im->launches += fip_bin_launches(geo) + 1;
   return call_leave(im, s);
 }
 
@@ -1434,6 +1436,7 @@ struct BatchSeq {
     b.count = count + k * ntiles;
     b.offset = offset + k * (ntiles + 1);
     b.cursor = cursor + k * ntiles;
+    b.base = nullptr;  // recounted: only grids too large for the joint binning
     b.entries = entries + k * cap;
     b.work = work + k * wcap;
     b.nwork = nwork + k;
@@ -1465,6 +1468,7 @@ struct fip_batch {
   size_t device_bytes = 0;
   int grid_ctas_per_sm = 0;
   float2* theta_tab = nullptr;  // theta terms of the pixel mapping (plain form)
+  unsigned* bin_base = nullptr; // binning scratch of a call (fip_launch_bin_batch)
   std::vector<BatchSeq> seq;
   unsigned* gather_err = nullptr;     // [1] set by a gather tile outside its domain
   cudaStream_t branch[kBranches] = {};
@@ -1496,6 +1500,7 @@ void batch_free(fip_batch* b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
   for (BatchSeq& q : b->seq) q.free_all();
   if (b->theta_tab) cudaFree(b->theta_tab);
+  if (b->bin_base) cudaFree(b->bin_base);
   if (b->gather_err) cudaFree(b->gather_err);
   for (int k = 0; k < kBranches; ++k) {
     if (b->branch[k]) cudaStreamDestroy(b->branch[k]);
@@ -1600,9 +1605,10 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
                         : cudaSuccess;
   };
   FIP_CUDA(phase(0));
-  // Per snapshot, on the branches: storage conversion and binning; the pixel
-  // mappings (plain form) on the low-priority mapping branches, joined only
-  // before the reprojections.
+  // Per snapshot, on the branches: storage conversion (and the binning of grids
+  // too large for the joint one, which runs on s); the pixel mappings (plain
+  // form) on the low-priority mapping branches, joined only before the
+  // reprojections.
   FIP_CUDA(cudaEventRecord(b->fork, s));
   for (int i = 0; i < kBranches; ++i) FIP_CUDA(cudaStreamWaitEvent(b->branch[i], b->fork, 0));
   if (!precise) {
@@ -1619,6 +1625,14 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
   }
   FipGridBatch in{};
   in.count = count;
+  FipBinBatch joint;
+  joint.count = 0;
+  for (int c = 0; c < nseq; ++c) {
+    const BatchSeq& q = b->seq[c];
+    if (l.per[c] == 0 || !fip_bin_batchable(q.geo)) continue;
+    FIP_CUDA(cudaMemsetAsync(q.count, 0, l.per[c] * q.ntiles * sizeof(unsigned), s));
+    FIP_CUDA(cudaMemsetAsync(q.bbox, 0, l.per[c] * 4 * sizeof(unsigned), s));
+  }
   for (int k = 0; k < count; ++k) {
     const BatchSeq& q = b->seq[l.sq[k]];
     const int j = l.loc[k];
@@ -1631,24 +1645,26 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
       launches += 1;
     }
     FipBins bins = q.bins(j);
-    FIP_CUDA(fip_launch_bin(q.geo, B[k], (int)nb[k], bins, bs));
-    launches += fip_bin_launches(q.geo);
+    if (fip_bin_batchable(q.geo)) {
+      joint.s[joint.count++] = fip_bin_snap(q.geo, B[k], (int)nb[k], bins,
+                                            q.grid + j * q.grid_elems);
+    } else {
+      FIP_CUDA(fip_launch_bin(q.geo, B[k], (int)nb[k], bins, q.grid + j * q.grid_elems, bs));
+      launches += fip_bin_launches(q.geo);
+    }
     in.s[k] = grid_snap(b, l, k, B[k], V[k], vr[k], vi[k]);
+  }
+  if (joint.count > 0) {
+    FIP_CUDA(fip_launch_bin_batch(joint, b->bin_base, s));
+    launches += 3;
   }
   for (int i = 0; i < kBranches; ++i) {
     FIP_CUDA(cudaEventRecord(b->join[i], b->branch[i]));
     FIP_CUDA(cudaStreamWaitEvent(s, b->join[i], 0));
   }
   FIP_CUDA(phase(1));
-  // One persistent gridding launch for the whole call (after each sequence's
-  // split tiles are zeroed), one batched transform per sequence.
-  for (int c = 0; c < nseq; ++c) {
-    const BatchSeq& q = b->seq[c];
-    if (l.per[c] == 0) continue;
-    FIP_CUDA(fip_launch_zero_batch(q.geo, q.multi, q.ntiles, q.nmulti, q.grid, q.grid_elems,
-                                   l.per[c], s));
-    launches += 1;
-  }
+  // One persistent gridding launch for the whole call, one batched transform
+  // per sequence.
   FIP_CUDA(fip_launch_grid_batch(in, vt, grid_compensated(precise, vt), s, b->grid_ctas_per_sm));
   launches += 1;
   FIP_CUDA(phase(2));
@@ -1881,6 +1897,20 @@ int fip_batch_create_sequences(fip_batch** out, const fip_imager_config* cfgs, s
   }
   if (b->cfg.form == FIP_FORM_PLAIN)
     FIP_BALLOC(dalloc(&b->theta_tab, fip_theta_table_elems(), tot));
+  {
+    size_t ntiles = 0, nbmax = 0;
+    for (const BatchSeq& q : b->seq)
+      if (fip_bin_batchable(q.geo)) {
+        ntiles = std::max(ntiles, q.ntiles);
+        nbmax = std::max(nbmax, q.cfg.max_baselines);
+      }
+    // ctas * count of a call: every snapshot takes at least one CTA.
+    const size_t rows = std::max<size_t>(
+        std::min<size_t>(FIP_MAX_BATCH, nseq * max_snapshots),
+        std::min<size_t>(kFipBinCtas,
+                         (size_t)fip_bin_ctas(1, nbmax) * nseq * max_snapshots));
+    if (ntiles) FIP_BALLOC(dalloc(&b->bin_base, rows * ntiles, tot));
+  }
   FIP_BALLOC(dalloc(&b->gather_err, 1, tot));
   FIP_BALLOC(cudaMemset(b->gather_err, 0, sizeof(unsigned)));
   {

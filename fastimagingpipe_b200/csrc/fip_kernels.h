@@ -19,6 +19,7 @@ struct FipBins {
   unsigned* count;    // [ntiles] entries per grid tile
   unsigned* offset;   // [ntiles + 1] exclusive scan of count
   unsigned* cursor;   // [ntiles] scatter cursors
+  unsigned* base;     // [fip_bin_ctas][ntiles] list positions per CTA, or null (recounted)
   unsigned* entries;  // [cap] (vis << 1 | mirrored), grouped by tile
   int4* work;         // [wcap] (tile, begin, end, single-chunk flag)
   unsigned* nwork;    // [1] number of work items
@@ -36,10 +37,24 @@ enum FipVisType { FIP_VIS_F32 = 0, FIP_VIS_F16 = 1, FIP_VIS_BF16 = 2, FIP_VIS_RA
 
 // ---- plain FP32 form (reference-faithful arithmetic, fip_plain.cu) ----
 cudaError_t fip_launch_taper(float* taper, const FipGeom& geo, cudaStream_t s);
+// Bins one snapshot; grid (or null): zero the tiles split over several work
+// items in it, as the gridding needs.
 cudaError_t fip_launch_bin(const FipGeom& geo, const float* B, int nb, FipBins& bins,
-                           cudaStream_t s);
+                           float2* grid, cudaStream_t s);
+// Bins the snapshots of `in` (geometries may differ; every ntiles within
+// fip_bin_batchable) in three launches.  Their counts and bbox are zero on
+// entry.  base: [fip_bin_ctas(in.count, ...) * in.count][max ntiles] scratch.
+bool fip_bin_batchable(const FipGeom& geo);
+FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBins& bins,
+                        float2* grid);
+cudaError_t fip_launch_bin_batch(FipBinBatch& in, unsigned* base, cudaStream_t s);
+// CTAs per snapshot of a binning launch over `count` snapshots of up to
+// nbmax visibilities; ctas * count <= kFipBinCtas.
+constexpr int kFipBinCtas = 296;
+int fip_bin_ctas(int count, size_t nbmax);
 // Kernels fip_launch_bin launches for nb > 0.
 int fip_bin_launches(const FipGeom& geo);
+// The binning has zeroed the grid's split tiles.
 // ctas_per_sm: persistent gridder CTAs per SM (0 = the most that fit,
 // fip_grid_max_ctas_per_sm).
 // vis_type FIP_VIS_RAW: vr, vi unused, the samples are *raw.
@@ -48,11 +63,6 @@ cudaError_t fip_launch_grid(const FipGeom& geo, const float* B, const void* vr, 
                             const FipBins& bins, float2* grid, int compensated, cudaStream_t s,
                             int ctas_per_sm = 0, const FipRawVis* raw = nullptr);
 int fip_grid_max_ctas_per_sm(int compensated);
-// Zeroes the split tiles of `count` snapshots of one geometry (their grids
-// and split-tile lists at base + k * stride) before a batched gridding launch.
-cudaError_t fip_launch_zero_batch(const FipGeom& geo, const unsigned* multi, size_t multi_stride,
-                                  const unsigned* nmulti, float2* grid, size_t grid_stride,
-                                  int count, cudaStream_t s);
 // One persistent gridding launch over the work items of all the batch's
 // snapshots (in.s[k]: inputs, bins, grid and geometry of snapshot k).
 cudaError_t fip_launch_grid_batch(const FipGridBatch& in, int vis_type, int compensated,

@@ -133,7 +133,7 @@ extern "C" int fip_grid_snapshot_noalloc(const float* vis_re, const float* vis_i
   bins.cap = kMaxEntries;
   bins.wcap = kMaxWork;
 
-  cudaError_t e = fip_launch_bin(geo, B, (int)nb, bins, s);
+  cudaError_t e = fip_launch_bin(geo, B, (int)nb, bins, reinterpret_cast<float2*>(grid), s);
   if (e == cudaSuccess)
     e = fip_launch_grid(geo, B, vis_re, vis_im, FIP_VIS_F32, nullptr, V, (int)nb, bins,
                         reinterpret_cast<float2*>(grid), 0, s);

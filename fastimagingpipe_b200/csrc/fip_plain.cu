@@ -69,15 +69,23 @@ struct Footprint {
   int a0, a1, b0, b1;
 };
 
-__device__ __forceinline__ bool footprint(const float* B, int v, float scale, int g, Footprint& f) {
-  const int hs = FIP_SUPPORT / 2;
-  const long gmin = -(long)g / 2, gmax = ((long)g - 1) / 2;
-  f.p1 = B[2 * v + 0] * scale;
-  f.p2 = B[2 * v + 1] * scale;
-  long a0 = max(fipref::ceil_l(f.p1 - hs), gmin), a1 = min(fipref::floor_l(f.p1 + hs), gmax);
-  long b0 = max(fipref::ceil_l(f.p2 - hs), gmin), b1 = min(fipref::floor_l(f.p2 + hs), gmax);
-  f.a0 = (int)a0; f.a1 = (int)a1; f.b0 = (int)b0; f.b1 = (int)b1;
-  return !(a0 > a1 || b0 > b1);
+// Positions beyond 1e9 cells (and NaN) have no footprint; the rest convert
+// exactly to 32-bit integers.
+__device__ __forceinline__ bool footprint(float b0, float b1, float scale, int g, Footprint& f) {
+  const float hs = (float)(FIP_SUPPORT / 2);
+  const int gmin = -(g / 2), gmax = (g - 1) / 2;
+  f.p1 = b0 * scale;
+  f.p2 = b1 * scale;
+  if (!(fabsf(f.p1) < 1e9f && fabsf(f.p2) < 1e9f)) {
+    f.a0 = f.b0 = 0;
+    f.a1 = f.b1 = -1;
+    return false;
+  }
+  f.a0 = max((int)ceilf(f.p1 - hs), gmin);
+  f.a1 = min((int)floorf(f.p1 + hs), gmax);
+  f.b0 = max((int)ceilf(f.p2 - hs), gmin);
+  f.b1 = min((int)floorf(f.p2 + hs), gmax);
+  return f.a0 <= f.a1 && f.b0 <= f.b1;
 }
 
 // Half-plane image of a virtual visibility.  The grid holds the Hermitian
@@ -150,7 +158,7 @@ __global__ void k_bin(const float* __restrict__ B, int nb, float scale, int g, i
                       unsigned* bbox) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   Footprint f;
-  bool ok = v < nb && footprint(B, v, scale, g, f);
+  bool ok = v < nb && footprint(B[2 * v], B[2 * v + 1], scale, g, f);
   unsigned k1 = 0, k2 = 0;
   if (ok) k1 = (unsigned)max(abs(f.a0), abs(f.a1));
   for (int mir = 0; mir < 2; ++mir) {
@@ -283,35 +291,71 @@ __global__ void __launch_bounds__(kScanThreads) k_bin_scan(
 
 // ---------------------------------------------------------------------------
 // Binning with per-CTA shared-memory histograms (grids of up to
-// kMaxSmemTiles tiles).  Each CTA takes a contiguous range of visibilities,
-// counts their tile entries in shared memory (native integer atomics, one
-// per entry: the hardware serialises lanes that hit one counter, cheaper
-// than matching the lanes first), and adds its non-zero counts to the global
-// ones; one CTA then scans the tiles.  The scatter pass recounts its range,
-// reserves one slice of each tile's list with one global atomic per
-// (CTA, tile), and fills it through shared-memory cursors.
+// kMaxSmemTiles tiles), the snapshots of a call side by side (blockIdx.y).
+// Each CTA takes a contiguous range of visibilities, counts their tile
+// entries in shared memory (native integer atomics, one per entry: the
+// hardware serialises lanes that hit one counter, cheaper than matching the
+// lanes first), and adds its non-zero counts to the global ones, which
+// returns where its entries start within each tile's list; one CTA per
+// snapshot then scans the tiles; the scatter pass starts its shared-memory
+// cursors from the two and fills the lists in one sweep.  Two CTAs per SM
+// over the whole launch: more of them multiply the histograms' fixed cost
+// (zeroing and merging every tile's counter), fewer leave the loads' latency
+// exposed.
+// Bound: the entries' integer arithmetic, then latency (three dependent
+// launches).  1.05 M visibilities at 2048^2: 25 + 11 + 50 us (count, scan,
+// scatter) with a recount in the scatter pass, 1,184 small CTAs and 64-bit
+// footprint arithmetic, 16 + 8 + 19 us (the split tiles' zeroing included,
+// a launch of its own before) in this form; eight snapshots of 0.45 M at
+// 2048^2 435 -> 108 us of kernels.
 // ---------------------------------------------------------------------------
-constexpr int kBinThreads = 256;
+constexpr int kBinThreads = 512;
+constexpr int kBinUnroll = 4;         // visibilities in flight per thread
 constexpr int kMaxSmemTiles = 12288;  // 48 KB of counters
 
-// Visits every tile entry (tile, code) of visibility v (ok = v is valid).
+// Visits the tile of every entry of a visibility at (b0, b1): f(tile, mir).
+// A footprint's nine rows and columns touch two tile rows and columns at
+// most, or the rows of both grid ends where it wraps.
 template <class F>
-__device__ __forceinline__ void for_each_entry(const float* B, int v, bool ok, float scale, int g,
+__device__ __forceinline__ void for_each_entry(float b0, float b1, float scale, int g,
                                                int tiles_c, unsigned& k1, unsigned& k2, F&& f) {
   Footprint fp;
-  ok = ok && footprint(B, v, scale, g, fp);
-  if (ok) k1 = max(k1, (unsigned)max(abs(fp.a0), abs(fp.a1)));
+  if (!footprint(b0, b1, scale, g, fp)) return;
+  k1 = max(k1, (unsigned)max(abs(fp.a0), abs(fp.a1)));
+#pragma unroll
   for (int mir = 0; mir < 2; ++mir) {
-    int c0 = 0, c1 = -1, trs[3], ntr = 0;
-    const bool on = ok && half_cols(fp, mir, g, c0, c1);
-    if (on) {
-      ntr = tile_rows(fp, mir, g, trs);
-      k2 = max(k2, (unsigned)c1);
+    int c0, c1;
+    if (!half_cols(fp, mir, g, c0, c1)) continue;
+    k2 = max(k2, (unsigned)c1);
+    const int rl = wrap_row(mir ? -fp.a1 : fp.a0, g), rh = wrap_row(mir ? -fp.a0 : fp.a1, g);
+    const int t0 = rl / FIP_GTILE, t1 = (rl <= rh ? rh : g - 1) / FIP_GTILE;
+    const int tc0 = c0 / FIP_GTILE, tc1 = c1 / FIP_GTILE;
+    for (int tr = t0; tr <= t1; ++tr)
+      for (int tc = tc0; tc <= tc1; ++tc) f((unsigned)(tr * tiles_c + tc), mir);
+    if (rl > rh && t0 > 0)  // wrapped: the rows from 0 (a one-tile grid has them already)
+      for (int tc = tc0; tc <= tc1; ++tc) f((unsigned)tc, mir);
+  }
+}
+
+// Runs body(b0, b1, v) over the CTA's visibilities, kBinUnroll loads in
+// flight per thread.
+template <class F>
+__device__ __forceinline__ void for_each_vis(const float* __restrict__ B, int v0, int v1,
+                                             F&& body) {
+  const bool pair = (reinterpret_cast<uintptr_t>(B) & 7) == 0;
+  for (int base = v0; base < v1; base += kBinThreads * kBinUnroll) {
+    float2 b[kBinUnroll];
+#pragma unroll
+    for (int q = 0; q < kBinUnroll; ++q) {
+      const int v = base + q * kBinThreads + threadIdx.x;
+      if (v < v1)
+        b[q] = pair ? reinterpret_cast<const float2*>(B)[v] : make_float2(B[2 * v], B[2 * v + 1]);
     }
-    const int tc0 = on ? c0 / FIP_GTILE : 0, tc1 = on ? c1 / FIP_GTILE : -1;
-    for (int kr = 0; kr < ntr; ++kr)
-      for (int tc = tc0; tc <= tc1; ++tc)
-        f((unsigned)(trs[kr] * tiles_c + tc), ((unsigned)v << 1) | (unsigned)mir);
+#pragma unroll
+    for (int q = 0; q < kBinUnroll; ++q) {
+      const int v = base + q * kBinThreads + threadIdx.x;
+      if (v < v1) body(b[q].x, b[q].y, v);
+    }
   }
 }
 
@@ -356,49 +400,99 @@ __device__ __forceinline__ uint3 block_scan3(uint3 v, uint3& total) {
   return make_uint3(base.x + inc.x - v.x, base.y + inc.y - v.y, base.z + inc.z - v.z);
 }
 
-// Tile scan run by one CTA of NT threads: offsets, cursors, the work list
-// (every band tile gets >= 1 item) and the list of tiles split over several
-// items.  cnt_s: the tile counts; wp_s: [ntiles + 1] scratch for the work
-// prefix (both shared memory).  The work items are written in a second,
-// parallel sweep (one thread per item, its tile found by bisection), so a
-// tile with thousands of entries does not serialise on one thread.
-template <int NT>
-__device__ __forceinline__ void scan_tiles(const unsigned* cnt_s, unsigned* wp_s,
-                                           const unsigned* bbox, int ntiles, int tiles_c, int g,
-                                           int layout, unsigned* offset, unsigned* cursor,
-                                           int4* work, unsigned* nwork, int wcap,
-                                           unsigned* multi, unsigned* nmulti) {
-  constexpr int PER = 8;
+// Count pass: per-CTA shared-memory counts added to count[] (base: the CTA's
+// start within each tile's list), and the occupied band (bbox[0], bbox[1]).
+// count and bbox are zero on entry.
+__global__ void __launch_bounds__(kBinThreads) k_bin_count(
+    const __grid_constant__ FipBinBatch in) {
+  extern __shared__ unsigned s_hist[];
+  __shared__ unsigned s_k[2];
+  const FipBinSnap& sn = in.s[blockIdx.y];
+  const int ntiles = sn.ntiles, g = sn.g, tiles_c = sn.tiles_c;
+  const float scale = sn.scale;
+  for (int t = threadIdx.x; t < ntiles; t += kBinThreads) s_hist[t] = 0;
+  if (threadIdx.x < 2) s_k[threadIdx.x] = 0;
+  __syncthreads();
+  const int per_cta = (sn.nb + gridDim.x - 1) / gridDim.x;
+  const int v0 = min(sn.nb, (int)blockIdx.x * per_cta), v1 = min(sn.nb, v0 + per_cta);
+  unsigned k1 = 0, k2 = 0;
+  for_each_vis(sn.B, v0, v1, [&](float b0, float b1, int) {
+    for_each_entry(b0, b1, scale, g, tiles_c, k1, k2,
+                   [&](unsigned tile, int) { atomicAdd(&s_hist[tile], 1u); });
+  });
+  k1 = __reduce_max_sync(0xffffffffu, k1);
+  k2 = __reduce_max_sync(0xffffffffu, k2);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&s_k[0], k1);
+    atomicMax(&s_k[1], k2);
+  }
+  __syncthreads();
+  if (sn.base) {
+    unsigned* base = sn.base + (size_t)blockIdx.x * ntiles;
+    for (int t = threadIdx.x; t < ntiles; t += kBinThreads)
+      if (s_hist[t]) base[t] = atomicAdd(&sn.count[t], s_hist[t]);
+  } else {
+    for (int t = threadIdx.x; t < ntiles; t += kBinThreads)
+      if (s_hist[t]) atomicAdd(&sn.count[t], s_hist[t]);
+  }
+  if (threadIdx.x == 0) {
+    atomicMax(&sn.bbox[0], s_k[0]);
+    atomicMax(&sn.bbox[1], s_k[1]);
+  }
+}
+
+// Tile scan over the final counts, one CTA of kScanThreads per snapshot:
+// offsets, cursors, the work list (every band tile gets >= 1 item) and the
+// list of tiles split over several items.  A thread scans kScanPer
+// consecutive tiles and writes their first work items; the split tiles'
+// further items are written by a warp per tile in a second sweep, so a tile
+// with thousands of entries does not serialise on one thread.
+constexpr int kScanPer = 8;
+__global__ void __launch_bounds__(kScanThreads) k_bin_scan_tiles(
+    const __grid_constant__ FipBinBatch in) {
+  extern __shared__ unsigned s_wp[];  // [ntiles] first work item of each split tile
+  const FipBinSnap& sn = in.s[blockIdx.x];
+  const int ntiles = sn.ntiles, tiles_c = sn.tiles_c, g = sn.g;
+  const unsigned wcap = sn.wcap;
+  const int k1 = (int)sn.bbox[0], k2 = (int)sn.bbox[1];
+  const bool full = sn.layout == 0;
   uint3 carry = make_uint3(0, 0, 0);
-  for (int base = 0; base < ntiles; base += NT * PER) {
-    const int t0 = base + threadIdx.x * PER;
-    unsigned c[PER], nch[PER];
-    uint3 sum = make_uint3(0, 0, 0);
+  for (int base = 0; base < ntiles; base += kScanThreads * kScanPer) {
+    const int t0 = base + threadIdx.x * kScanPer;
+    unsigned c[kScanPer], nch[kScanPer];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int t = t0 + k;
-      c[k] = 0;
-      nch[k] = 0;
-      if (t < ntiles) {
-        c[k] = cnt_s[t];
-        nch[k] = in_band(t, tiles_c, g, layout, bbox) ? max(1u, (c[k] + FIP_GCHUNK - 1) / FIP_GCHUNK)
-                                                      : 0u;
+    for (int k = 0; k < kScanPer; ++k) c[k] = t0 + k < ntiles ? sn.count[t0 + k] : 0u;
+    uint3 sum = make_uint3(0, 0, 0);
+    int tr = t0 / tiles_c, tc = t0 - tr * tiles_c;
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) {
+      const int r0 = tr * FIP_GTILE, r1 = min(r0 + FIP_GTILE, g) - 1;
+      const bool band = full || (tc * FIP_GTILE <= k2 && (r0 <= k1 || r1 >= g - k1));
+      nch[k] = t0 + k < ntiles && band ? max(1u, (c[k] + FIP_GCHUNK - 1) / FIP_GCHUNK) : 0u;
+      if (++tc == tiles_c) {
+        tc = 0;
+        ++tr;
       }
       sum.x += c[k];
       sum.y += nch[k];
       sum.z += nch[k] > 1 ? 1u : 0u;
     }
     uint3 total;
-    const uint3 ex = block_scan3<NT>(sum, total);
+    const uint3 ex = block_scan3<kScanThreads>(sum, total);
     unsigned run = carry.x + ex.x, wrun = carry.y + ex.y, mrun = carry.z + ex.z;
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
+    for (int k = 0; k < kScanPer; ++k) {
       const int t = t0 + k;
       if (t < ntiles) {
-        offset[t] = run;
-        cursor[t] = 0;
-        wp_s[t] = wrun;
-        if (nch[k] > 1) multi[mrun++] = (unsigned)t;
+        sn.offset[t] = run;
+        if (!sn.base) sn.cursor[t] = 0;
+        if (nch[k] > 0 && wrun < wcap)
+          sn.work[wrun] = make_int4(t, (int)run, (int)(run + min((unsigned)FIP_GCHUNK, c[k])),
+                                    nch[k] == 1);
+        if (nch[k] > 1) {
+          sn.multi[mrun++] = (unsigned)t;
+          s_wp[t] = wrun;
+        }
         run += c[k];
         wrun += nch[k];
       }
@@ -408,101 +502,18 @@ __device__ __forceinline__ void scan_tiles(const unsigned* cnt_s, unsigned* wp_s
     carry.z += total.z;
   }
   if (threadIdx.x == 0) {
-    offset[ntiles] = carry.x;
-    wp_s[ntiles] = carry.y;
-    *nwork = min(carry.y, (unsigned)wcap);
-    *nmulti = carry.z;
+    sn.offset[ntiles] = carry.x;
+    *sn.nwork = min(carry.y, wcap);
+    *sn.nmulti = carry.z;
   }
   __syncthreads();
-  const unsigned nw = min(carry.y, (unsigned)wcap);
-  for (unsigned w = threadIdx.x; w < nw; w += NT) {
-    int lo = 0, hi = ntiles - 1;  // last tile with wp_s[t] <= w
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (wp_s[mid] <= w) lo = mid; else hi = mid - 1;
-    }
-    const int t = lo;
-    const unsigned q = w - wp_s[t], nch = wp_s[t + 1] - wp_s[t], c = cnt_s[t];
-    const unsigned run = offset[t];
-    work[w] = make_int4(t, (int)(run + min(q * FIP_GCHUNK, c)),
-                        (int)(run + min((q + 1) * FIP_GCHUNK, c)), nch == 1);
-  }
-}
-
-// Count pass: per-CTA shared-memory counts added to count[], and the
-// occupied band (bbox[0], bbox[1]).  count and bbox are zero on entry.
-__global__ void __launch_bounds__(kBinThreads) k_bin_count(
-    const float* __restrict__ B, int nb, int per_cta, float scale, int g, int tiles_c, int ntiles,
-    unsigned* count, unsigned* bbox) {
-  extern __shared__ unsigned s_hist[];
-  __shared__ unsigned s_k[2];
-  for (int t = threadIdx.x; t < ntiles; t += kBinThreads) s_hist[t] = 0;
-  if (threadIdx.x < 2) s_k[threadIdx.x] = 0;
-  __syncthreads();
-  const int v0 = blockIdx.x * per_cta, v1 = min(nb, v0 + per_cta);
-  unsigned k1 = 0, k2 = 0;
-  for (int base = v0; base < v1; base += kBinThreads) {
-    const int v = base + threadIdx.x;
-    for_each_entry(B, v, v < v1, scale, g, tiles_c, k1, k2,
-                   [&](unsigned tile, unsigned) { atomicAdd(&s_hist[tile], 1u); });
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    k1 = max(k1, __shfl_xor_sync(0xffffffffu, k1, o));
-    k2 = max(k2, __shfl_xor_sync(0xffffffffu, k2, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(&s_k[0], k1);
-    atomicMax(&s_k[1], k2);
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < ntiles; t += kBinThreads)
-    if (s_hist[t]) atomicAdd(&count[t], s_hist[t]);
-  if (threadIdx.x == 0) {
-    atomicMax(&bbox[0], s_k[0]);
-    atomicMax(&bbox[1], s_k[1]);
-  }
-}
-
-// Tile scan over the final counts, one CTA of kScanThreads.
-__global__ void __launch_bounds__(kScanThreads) k_bin_scan_tiles(
-    const unsigned* __restrict__ count, const unsigned* __restrict__ bbox, int ntiles,
-    int tiles_c, int g, int layout, unsigned* offset, unsigned* cursor, int4* work,
-    unsigned* nwork, int wcap, unsigned* multi, unsigned* nmulti) {
-  extern __shared__ unsigned s_cnt[];  // [ntiles] counts, then [ntiles + 1] work prefix
-  __shared__ unsigned s_k[2];
-  for (int t = threadIdx.x; t < ntiles; t += kScanThreads) s_cnt[t] = count[t];
-  if (threadIdx.x < 2) s_k[threadIdx.x] = bbox[threadIdx.x];
-  __syncthreads();
-  scan_tiles<kScanThreads>(s_cnt, s_cnt + ntiles, s_k, ntiles, tiles_c, g, layout, offset,
-                           cursor, work, nwork, wcap, multi, nmulti);
-}
-
-// Scatter pass: entries of the CTA's visibility range into the tile lists.
-__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(
-    const float* __restrict__ B, int nb, int per_cta, float scale, int g, int tiles_c, int ntiles,
-    const unsigned* __restrict__ offset, unsigned* cursor, unsigned* entries) {
-  extern __shared__ unsigned s_hist[];
-  for (int t = threadIdx.x; t < ntiles; t += kBinThreads) s_hist[t] = 0;
-  __syncthreads();
-  const int v0 = blockIdx.x * per_cta, v1 = min(nb, v0 + per_cta);
-  unsigned k1 = 0, k2 = 0;
-  for (int base = v0; base < v1; base += kBinThreads) {
-    const int v = base + threadIdx.x;
-    for_each_entry(B, v, v < v1, scale, g, tiles_c, k1, k2,
-                   [&](unsigned tile, unsigned) { atomicAdd(&s_hist[tile], 1u); });
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < ntiles; t += kBinThreads) {
-    const unsigned c = s_hist[t];
-    if (c) s_hist[t] = offset[t] + atomicAdd(&cursor[t], c);
-  }
-  __syncthreads();
-  for (int base = v0; base < v1; base += kBinThreads) {
-    const int v = base + threadIdx.x;
-    for_each_entry(B, v, v < v1, scale, g, tiles_c, k1, k2,
-                   [&](unsigned tile, unsigned code) {
-                     entries[atomicAdd(&s_hist[tile], 1u)] = code;
-                   });
+  for (unsigned m = threadIdx.x >> 5; m < carry.z; m += kScanThreads / 32) {
+    const unsigned t = sn.multi[m], run = sn.offset[t], c = sn.count[t], w0 = s_wp[t];
+    const unsigned n = (c + FIP_GCHUNK - 1) / FIP_GCHUNK;
+    for (unsigned q = 1 + (threadIdx.x & 31); q < n; q += 32)
+      if (w0 + q < wcap)
+        sn.work[w0 + q] = make_int4((int)t, (int)(run + q * FIP_GCHUNK),
+                                    (int)(run + min((q + 1) * FIP_GCHUNK, c)), 0);
   }
 }
 
@@ -510,25 +521,67 @@ __device__ __forceinline__ size_t cell_index(int row, int col, int g, int hp, in
   return layout ? (size_t)col * g + row : (size_t)row * hp + col;
 }
 
-// Zeroes the tiles that several work items reduce into.
-// Batched launches: snapshot blockIdx.y, its lists at multi + y * multi_stride,
-// nmulti[y], its grid at grid + y * grid_stride.
-__global__ void k_zero_tiles(const unsigned* __restrict__ multi, const unsigned* __restrict__ nmulti,
-                             int tiles_c, int g, int hp, int layout, float2* __restrict__ grid,
-                             size_t multi_stride, size_t grid_stride) {
-  multi += blockIdx.y * multi_stride;
-  grid += blockIdx.y * grid_stride;
-  const unsigned nm = nmulti[blockIdx.y];
-  for (unsigned w = blockIdx.x; w < nm; w += gridDim.x) {
-    const int t = (int)multi[w];
-    const int row0 = (t / tiles_c) * FIP_GTILE, col0 = (t % tiles_c) * FIP_GTILE;
-    for (int k = threadIdx.x; k < FIP_GTILE * FIP_GTILE; k += kThreads) {
-      const int lr = layout ? k % FIP_GTILE : k / FIP_GTILE;
-      const int lc = layout ? k / FIP_GTILE : k % FIP_GTILE;
-      const int row = row0 + lr, col = col0 + lc;
-      if (row < g && col < hp) grid[cell_index(row, col, g, hp, layout)] = make_float2(0.f, 0.f);
+// Zeroes grid tile t (the CTA's threads together).
+__device__ __forceinline__ void zero_tile(int t, int tiles_c, int g, int hp, int layout,
+                                          float2* __restrict__ grid, int threads) {
+  const int row0 = (t / tiles_c) * FIP_GTILE, col0 = (t % tiles_c) * FIP_GTILE;
+  for (int k = threadIdx.x; k < FIP_GTILE * FIP_GTILE; k += threads) {
+    const int lr = layout ? k % FIP_GTILE : k / FIP_GTILE;
+    const int lc = layout ? k / FIP_GTILE : k % FIP_GTILE;
+    const int row = row0 + lr, col = col0 + lc;
+    if (row < g && col < hp) grid[cell_index(row, col, g, hp, layout)] = make_float2(0.f, 0.f);
+  }
+}
+
+// Scatter pass: entries of the CTA's visibility range into the tile lists,
+// and the split tiles of the grid zeroed (their work items reduce into them).
+// Without the count pass's list positions (base) the range is recounted and
+// reserves its slices from the cursors.
+__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(
+    const __grid_constant__ FipBinBatch in) {
+  extern __shared__ unsigned s_hist[];
+  const FipBinSnap& sn = in.s[blockIdx.y];
+  const int ntiles = sn.ntiles, g = sn.g, tiles_c = sn.tiles_c;
+  const float scale = sn.scale;
+  const int per_cta = (sn.nb + gridDim.x - 1) / gridDim.x;
+  const int v0 = min(sn.nb, (int)blockIdx.x * per_cta), v1 = min(sn.nb, v0 + per_cta);
+  unsigned k1 = 0, k2 = 0;
+  if (sn.base) {
+    const unsigned* base = sn.base + (size_t)blockIdx.x * ntiles;
+    for (int t = threadIdx.x; t < ntiles; t += kBinThreads) s_hist[t] = sn.offset[t] + base[t];
+  } else {
+    for (int t = threadIdx.x; t < ntiles; t += kBinThreads) s_hist[t] = 0;
+    __syncthreads();
+    for_each_vis(sn.B, v0, v1, [&](float b0, float b1, int) {
+      for_each_entry(b0, b1, scale, g, tiles_c, k1, k2,
+                     [&](unsigned tile, int) { atomicAdd(&s_hist[tile], 1u); });
+    });
+    __syncthreads();
+    for (int t = threadIdx.x; t < ntiles; t += kBinThreads) {
+      const unsigned c = s_hist[t];
+      if (c) s_hist[t] = sn.offset[t] + atomicAdd(&sn.cursor[t], c);
     }
   }
+  __syncthreads();
+  for_each_vis(sn.B, v0, v1, [&](float b0, float b1, int v) {
+    for_each_entry(b0, b1, scale, g, tiles_c, k1, k2, [&](unsigned tile, int mir) {
+      sn.entries[atomicAdd(&s_hist[tile], 1u)] = ((unsigned)v << 1) | (unsigned)mir;
+    });
+  });
+  if (sn.grid) {
+    const unsigned nm = *sn.nmulti;
+    for (unsigned m = blockIdx.x; m < nm; m += gridDim.x)
+      zero_tile((int)sn.multi[m], tiles_c, g, sn.hp, sn.layout, sn.grid, kBinThreads);
+  }
+}
+
+// The split tiles of a snapshot whose grid has too many tiles for the
+// binning above.
+__global__ void k_zero_tiles(const unsigned* __restrict__ multi, const unsigned* __restrict__ nmulti,
+                             int tiles_c, int g, int hp, int layout, float2* __restrict__ grid) {
+  const unsigned nm = *nmulti;
+  for (unsigned w = blockIdx.x; w < nm; w += gridDim.x)
+    zero_tile((int)multi[w], tiles_c, g, hp, layout, grid, kThreads);
 }
 
 template <int VT>
@@ -570,7 +623,7 @@ __device__ __forceinline__ void entry_taps(const float* __restrict__ B, const vo
                                            int tcol0, const FipRawVis& raw, EntryTaps& e) {
   const int v = (int)(ent >> 1), mir = (int)(ent & 1);
   Footprint f;
-  footprint(B, v, scale, g, f);
+  footprint(B[2 * v], B[2 * v + 1], scale, g, f);
   int c0, c1;
   half_cols(f, mir, g, c0, c1);
   // Visibility weighting (FIPkernels.cu:188-195).
@@ -2203,36 +2256,74 @@ cudaError_t fip_launch_taper(float* taper, const FipGeom& geo, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-int fip_bin_launches(const FipGeom&) { return 3; }
+bool fip_bin_batchable(const FipGeom& geo) {
+  return (size_t)geo.tiles_r * geo.tiles_c <= (size_t)kMaxSmemTiles;
+}
+
+int fip_bin_launches(const FipGeom& geo) { return fip_bin_batchable(geo) ? 3 : 4; }
+
+int fip_bin_ctas(int count, size_t nbmax) {
+  const size_t per = (size_t)kBinThreads;
+  return std::max(1, (int)std::min<size_t>(kFipBinCtas / std::max(1, count),
+                                           (nbmax + per - 1) / per));
+}
+
+FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBins& bins,
+                        float2* grid) {
+  FipBinSnap q{};
+  q.B = B;
+  q.nb = nb;
+  q.scale = geo.cell * (float)(size_t)geo.g;  // r1r2_scale (FIPkernels.cu:584)
+  q.g = geo.g;
+  q.hp = geo.hp;
+  q.tiles_c = geo.tiles_c;
+  q.ntiles = geo.tiles_r * geo.tiles_c;
+  q.layout = geo.layout;
+  q.wcap = (unsigned)bins.wcap;
+  q.count = bins.count;
+  q.offset = bins.offset;
+  q.cursor = bins.cursor;
+  q.entries = bins.entries;
+  q.work = bins.work;
+  q.nwork = bins.nwork;
+  q.bbox = bins.bbox;
+  q.multi = bins.multi;
+  q.nmulti = bins.nmulti;
+  q.grid = grid;
+  return q;
+}
+
+cudaError_t fip_launch_bin_batch(FipBinBatch& in, unsigned* base, cudaStream_t s) {
+  if (in.count < 1 || in.count > FIP_MAX_BATCH) return cudaErrorInvalidValue;
+  int ntiles = 0, nb = 0;
+  for (int k = 0; k < in.count; ++k) {
+    ntiles = std::max(ntiles, in.s[k].ntiles);
+    nb = std::max(nb, in.s[k].nb);
+  }
+  if (ntiles > kMaxSmemTiles) return cudaErrorInvalidValue;
+  const int ctas = fip_bin_ctas(in.count, (size_t)nb);
+  for (int k = 0; k < in.count; ++k)
+    in.s[k].base = base ? base + (size_t)k * ctas * ntiles : nullptr;
+  const size_t smem = (size_t)ntiles * sizeof(unsigned);
+  const dim3 grid(ctas, in.count);
+  k_bin_count<<<grid, kBinThreads, smem, s>>>(in);
+  k_bin_scan_tiles<<<in.count, kScanThreads, smem, s>>>(in);
+  k_bin_scatter<<<grid, kBinThreads, smem, s>>>(in);
+  return cudaGetLastError();
+}
 
 cudaError_t fip_launch_bin(const FipGeom& geo, const float* B, int nb, FipBins& bins,
-                           cudaStream_t s) {
+                           float2* grid, cudaStream_t s) {
   const int ntiles = geo.tiles_r * geo.tiles_c;
   const float scale = geo.cell * (float)(size_t)geo.g;  // r1r2_scale (FIPkernels.cu:584)
   cudaError_t e = cudaMemsetAsync(bins.count, 0, ntiles * sizeof(unsigned), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(bins.bbox, 0, 4 * sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
-  if (ntiles <= kMaxSmemTiles) {
-    const int cta = max(1, min(8 * sm_count(), (nb + kBinThreads - 1) / kBinThreads));
-    const int per_cta = (nb + cta - 1) / cta;
-    const size_t smem = (size_t)ntiles * sizeof(unsigned);
-    if (nb > 0)
-      k_bin_count<<<cta, kBinThreads, smem, s>>>(B, nb, per_cta, scale, geo.g, geo.tiles_c,
-                                                  ntiles, bins.count, bins.bbox);
-    const size_t scan_smem = (2 * (size_t)ntiles + 1) * sizeof(unsigned);
-    cudaError_t ea = cudaFuncSetAttribute(k_bin_scan_tiles,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)((2 * (size_t)kMaxSmemTiles + 1) * sizeof(unsigned)));
-    if (ea != cudaSuccess) return ea;
-    k_bin_scan_tiles<<<1, kScanThreads, scan_smem, s>>>(bins.count, bins.bbox, ntiles, geo.tiles_c,
-                                                    geo.g, geo.layout, bins.offset, bins.cursor,
-                                                    bins.work, bins.nwork, (int)bins.wcap,
-                                                    bins.multi, bins.nmulti);
-    if (nb > 0)
-      k_bin_scatter<<<cta, kBinThreads, smem, s>>>(B, nb, per_cta, scale, geo.g, geo.tiles_c,
-                                                    ntiles, bins.offset, bins.cursor,
-                                                    bins.entries);
-    return cudaGetLastError();
+  if (fip_bin_batchable(geo)) {
+    FipBinBatch in;
+    in.count = 1;
+    in.s[0] = fip_bin_snap(geo, B, nb, bins, grid);
+    return fip_launch_bin_batch(in, bins.base, s);
   }
   const int blocks = (nb + kThreads - 1) / kThreads;
   if (nb > 0)
@@ -2244,6 +2335,9 @@ cudaError_t fip_launch_bin(const FipGeom& geo, const float* B, int nb, FipBins& 
   if (nb > 0)
     k_bin<1><<<blocks, kThreads, 0, s>>>(B, nb, scale, geo.g, geo.tiles_c, bins.cursor,
                                          bins.offset, bins.entries, nullptr);
+  if (grid)
+    k_zero_tiles<<<sm_count(), kThreads, 0, s>>>(bins.multi, bins.nmulti, geo.tiles_c, geo.g,
+                                                 geo.hp, geo.layout, grid);
   return cudaGetLastError();
 }
 
@@ -2259,8 +2353,6 @@ cudaError_t fip_launch_grid(const FipGeom& geo, const float* B, const void* vr, 
   const FipRawVis rv = raw ? *raw : FipRawVis{};
   const float scale = geo.cell * (float)(size_t)geo.g;
   const int sms = sm_count();
-  k_zero_tiles<<<sms, kThreads, 0, s>>>(bins.multi, bins.nmulti, geo.tiles_c, geo.g, geo.hp,
-                                        geo.layout, grid, 0, 0);
   const size_t smem = grid_smem_bytes(compensated != 0);
   const int most = fip_grid_max_ctas_per_sm(compensated);
   const int blocks = sms * (ctas_per_sm > 0 ? min(ctas_per_sm, most) : most);
@@ -2283,16 +2375,6 @@ cudaError_t fip_launch_grid(const FipGeom& geo, const float* B, const void* vr, 
   }
 #undef FIP_GRID_CASE
   (void)nb;
-  return cudaGetLastError();
-}
-
-cudaError_t fip_launch_zero_batch(const FipGeom& geo, const unsigned* multi, size_t multi_stride,
-                                  const unsigned* nmulti, float2* grid, size_t grid_stride,
-                                  int count, cudaStream_t s) {
-  if (count < 1 || count > 65535) return cudaErrorInvalidValue;
-  k_zero_tiles<<<dim3(sm_count(), count), kThreads, 0, s>>>(multi, nmulti, geo.tiles_c, geo.g,
-                                                            geo.hp, geo.layout, grid,
-                                                            multi_stride, grid_stride);
   return cudaGetLastError();
 }
 
