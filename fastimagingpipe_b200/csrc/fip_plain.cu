@@ -648,9 +648,10 @@ __device__ __forceinline__ void entry_taps(const float* __restrict__ B, const vo
   e.mir = mir;
   const int nr = f.a1 - f.a0 + 1, nc = c1 - c0 + 1;
   // Tap row ia is grid row wrap(r1), r1 = a0 + ia (mirrored: -(a0 + ia)).
-  // Unless the grid is one tile high, no tile holds the wrap point inside
-  // it (it falls on a tile edge), so a tile's rows of the footprint are one
-  // run of ia along which the tile row moves by +1 (mirrored: -1).
+  // Unless the grid is little more than one tile high (fewer than nine rows
+  // beyond it), no tile holds rows of a footprint from both grid ends, so a
+  // tile's rows of the footprint are one run of ia along which the tile row
+  // moves by +1 (mirrored: -1).
   int ia_lo = 9, ia_hi = 0, lr_first = 0;
 #pragma unroll
   for (int a = 0; a < 9; ++a)
@@ -772,12 +773,15 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
 #pragma unroll
     for (int a = 0; a < 9; ++a) {
       if (a < et.ia_lo || a >= et.ia_hi) continue;
-      // One tile row holding the whole grid may hold the wrap point: each
-      // tap row is then wrapped on its own.
-      const int rc = g > FIP_GTILE
-                         ? et.cell0 + (a - et.ia_lo) * dstep
-                         : (wrap_row(et.r1 + (et.mir ? et.ia_lo - a : a - et.ia_lo), g) - trow0) *
-                                   kTS + lc0;
+      // Grids of little more than one tile: a tile may hold rows from both
+      // grid ends, with the rows between them in another tile or none, so
+      // each tap row is wrapped and checked on its own.
+      int rc = et.cell0 + (a - et.ia_lo) * dstep;
+      if (g < FIP_GTILE + 9) {
+        const int lr = wrap_row(et.r1 + (et.mir ? et.ia_lo - a : a - et.ia_lo), g) - trow0;
+        if ((unsigned)lr >= (unsigned)FIP_GTILE) continue;
+        rc = lr * kTS + lc0;
+      }
       const float ra = wrf * et.k1[a], rb = wif * et.k1[a];
 #pragma unroll
       for (int b = 0; b < 9; ++b) {

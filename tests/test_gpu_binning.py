@@ -37,7 +37,7 @@ def grid64(vr, vi, B, V, n, cell):
     return ((full + neg.conj()) / 2)[:, :g // 2 + 1]
 
 
-@pytest.mark.parametrize("n", [16, 40, 100, 256, 1000])
+@pytest.mark.parametrize("n", [16, 40, 44, 48, 100, 256, 1000])
 @pytest.mark.parametrize("nb,offset", [(1, 0), (511, 1), (2048, 0), (5000, 1)])
 def test_binned_grid(cuda, n, nb, offset):
     import torch
