@@ -117,12 +117,24 @@ struct FipBinSnap {
   unsigned* multi;
   unsigned* nmulti;
   float2* grid;
+  unsigned* clear;  // (or null) a word the scan zeroes: the image's maximum
 };
 
-// The snapshots of one binning launch (a kernel parameter of about 8.2 KB).
+// The snapshots of one binning launch (a kernel parameter of about 8.7 KB).
 struct FipBinBatch {
   int count;
   FipBinSnap s[FIP_MAX_BATCH];
+};
+
+// The snapshots of one reprojection launch (one image size): the plane
+// bases, the visibility counts, the destination images and (or null) where
+// their maxima go.
+struct FipGatherBatch {
+  int count;
+  const float* V[FIP_MAX_BATCH];
+  int nb[FIP_MAX_BATCH];
+  float* dst[FIP_MAX_BATCH];
+  unsigned* img_max[FIP_MAX_BATCH];
 };
 
 // The snapshots of one batched gridding launch (a kernel parameter of

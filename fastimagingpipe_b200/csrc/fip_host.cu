@@ -269,6 +269,15 @@ struct Lane {
   bool plan_ok = false;
 };
 constexpr int kLanes = 3;
+// The largest image side whose multi-snapshot calls share launches.  Small
+// images leave most SMs idle and are bound by launches and by each kernel's
+// latency; large ones fill the device by themselves, and there the lanes'
+// overlap of one snapshot's latency-bound stages with another's
+// issue-bound ones wins.  Three-snapshot calls, lanes against shared launches,
+// us (plain / FP32 / FP16): 128^2 138 / 119 / 124 against 76 / 62 / 60, 512^2
+// 104 / 100 / 132 against 76 / 78 / 73, 1024^2 142 / 142 / 129 against
+// 137 / 135 / 124, 2048^2 348 / 312 / 265 against 354 / 326 / 280.
+constexpr int kMergedMax = 1024;
 
 struct fip_imager {
   fip_imager_config cfg{};
@@ -290,12 +299,19 @@ struct fip_imager {
   float2* twiddles = nullptr;        // e^{+2 pi i k / G}, k < G
   float2* theta_tab = nullptr;       // theta terms of the pixel mapping (plain form)
   float* taper = nullptr;            // N/2 + 1 taper values, N/2 + 1 reciprocals
+  // The lanes' scratch, each array's lanes side by side (lane l at l * stride),
+  // so that a call's snapshots can also share launches (image_merged).
   Lane lane[kLanes];
+  std::vector<void*> lane_mem;       // the arrays' allocations
+  size_t grid_stride = 0, col_stride = 0;
+  unsigned* zero_block = nullptr;    // the lanes' counts and bboxes, then fuse_count
+  size_t zero_words = 0;             // of which a merged call clears this many
   int lanes = 1;                     // lanes in use (kLanes with the pruned transform)
   int last_lane = 0;                 // lane of the last gridded snapshot
   cudaEvent_t ev_start = nullptr;    // start of a multi-snapshot call (lanes wait on it)
   cudaEvent_t ev_free[6] = {};       // sequence ring slot released by its last trigger
   float* images[6] = {};             // 0..2: one call's snapshots; all: the sequence ring
+                                     // (side by side, N*N apart)
   int ring = 3;                      // images allocated (6 with lanes)
   float* maxima = nullptr;           // [6] device floats (written as max bits)
   float* result = nullptr;           // U*U
@@ -374,19 +390,13 @@ static void imager_free(fip_imager* im) {
   for (Lane& L : im->lane) {
     if (L.stream) cudaStreamSynchronize(L.stream);
     if (L.plan_ok) cufftDestroy(L.plan);
-    void* lp[] = {L.grid, L.bins.count, L.bins.offset, L.bins.cursor, L.bins.base, L.bins.entries,
-                  L.bins.work, L.bins.nwork, L.bins.bbox, L.bins.multi, L.bins.nmulti,
-                  L.colbuf, L.pre, L.targets, L.q_re, L.q_im, L.q_scale};
-    for (void* p : lp)
-      if (p) cudaFree(p);
     if (L.ev_done) cudaEventDestroy(L.ev_done);
     if (L.ev_targets) cudaEventDestroy(L.ev_targets);
     if (L.stream) cudaStreamDestroy(L.stream);
   }
-  for (float* p : im->images)
-    if (p) cudaFree(p);
-  void* dptrs[] = {im->taper, im->twiddles, im->theta_tab, im->maxima, im->result, im->stats,
-                   im->d_snap, im->d_V, im->gather_err, im->fuse_count, im->fuse_stats};
+  for (void* p : im->lane_mem) cudaFree(p);
+  void* dptrs[] = {im->images[0], im->taper, im->twiddles, im->theta_tab, im->maxima, im->result, im->stats,
+                   im->d_snap, im->d_V, im->gather_err, im->fuse_stats};
   for (void* p : dptrs)
     if (p) cudaFree(p);
   void* hptrs[] = {im->h_snap, im->h_V, im->h_result, im->h_err};
@@ -535,27 +545,65 @@ int fip_imager_create(fip_imager** out, const fip_imager_config* cfg) {
     FIP_ALLOC(cudaStreamCreateWithPriority(&L.stream, cudaStreamNonBlocking, prio_greatest));
     FIP_ALLOC(cudaEventCreateWithFlags(&L.ev_done, cudaEventDisableTiming));
     FIP_ALLOC(cudaEventCreateWithFlags(&L.ev_targets, cudaEventDisableTiming));
-    FIP_ALLOC(dalloc(&L.grid, (size_t)geo.g * geo.hp, tot));
     L.bins.cap = 12 * nb;
     L.bins.wcap = ntiles + L.bins.cap / FIP_GCHUNK + 1;
-    FIP_ALLOC(dalloc(&L.bins.count, ntiles, tot));
-    FIP_ALLOC(dalloc(&L.bins.offset, ntiles + 1, tot));
-    FIP_ALLOC(dalloc(&L.bins.cursor, ntiles, tot));
-    if (fip_bin_batchable(geo))
-      FIP_ALLOC(dalloc(&L.bins.base, (size_t)fip_bin_ctas(1, nb) * ntiles, tot));
-    FIP_ALLOC(dalloc(&L.bins.entries, L.bins.cap, tot));
-    FIP_ALLOC(dalloc(&L.bins.work, L.bins.wcap, tot));
-    FIP_ALLOC(dalloc(&L.bins.nwork, 1, tot));
-    FIP_ALLOC(dalloc(&L.bins.bbox, 4, tot));
-    FIP_ALLOC(dalloc(&L.bins.multi, ntiles, tot));
-    FIP_ALLOC(dalloc(&L.bins.nmulti, 1, tot));
-    FIP_ALLOC(dalloc(&L.pre, n2, tot));
-    if (cfg->form == FIP_FORM_PLAIN && cfg->reproject == 0) FIP_ALLOC(dalloc(&L.targets, n2, tot));
-    if (im->custom_fft) FIP_ALLOC(dalloc(&L.colbuf, (size_t)geo.hp * geo.n, tot));
-    if (cfg->form == FIP_FORM_PRECISE && cfg->vis_storage != FIP_STORE_F32) {
-      FIP_ALLOC(dalloc((uint16_t**)&L.q_re, nb, tot));
-      FIP_ALLOC(dalloc((uint16_t**)&L.q_im, nb, tot));
-      FIP_ALLOC(dalloc(&L.q_scale, fip_qblocks(nb), tot));
+  }
+  // Every lane's `member`, `count` elements each, from one allocation.
+#define FIP_LANES(member, count)                                            \
+  do {                                                                      \
+    decltype(im->lane[0].member) base_ = nullptr;                           \
+    const size_t n_ = (count);                                              \
+    FIP_ALLOC(dalloc(&base_, n_ * im->lanes, tot));                         \
+    im->lane_mem.push_back(base_);                                          \
+    for (int l_ = 0; l_ < im->lanes; ++l_) im->lane[l_].member = base_ + l_ * n_; \
+  } while (0)
+  // Strides in whole 512-byte blocks keep every lane's grid and column buffer
+  // as aligned as an allocation of its own.
+  im->grid_stride = ((size_t)geo.g * geo.hp + 63) / 64 * 64;
+  im->col_stride = ((size_t)geo.hp * geo.n + 63) / 64 * 64;
+  FIP_LANES(grid, im->grid_stride);
+  FIP_LANES(bins.offset, ntiles + 1);
+  FIP_LANES(bins.cursor, ntiles);
+  if (fip_bin_batchable(geo)) FIP_LANES(bins.base, (size_t)fip_bin_ctas(1, nb) * ntiles);
+  FIP_LANES(bins.entries, im->lane[0].bins.cap);
+  FIP_LANES(bins.work, im->lane[0].bins.wcap);
+  FIP_LANES(bins.nwork, 1);
+  FIP_LANES(bins.multi, ntiles);
+  FIP_LANES(bins.nmulti, 1);
+  FIP_LANES(pre, n2);
+  if (cfg->form == FIP_FORM_PLAIN && cfg->reproject == 0) FIP_LANES(targets, n2);
+  if (im->custom_fft) FIP_LANES(colbuf, im->col_stride);
+  if (cfg->form == FIP_FORM_PRECISE && cfg->vis_storage != FIP_STORE_F32) {
+    uint16_t *qr = nullptr, *qi = nullptr;
+    FIP_ALLOC(dalloc(&qr, nb * im->lanes, tot));
+    im->lane_mem.push_back(qr);
+    FIP_ALLOC(dalloc(&qi, nb * im->lanes, tot));
+    im->lane_mem.push_back(qi);
+    for (int l = 0; l < im->lanes; ++l) {
+      im->lane[l].q_re = qr + l * nb;
+      im->lane[l].q_im = qi + l * nb;
+    }
+    FIP_LANES(q_scale, fip_qblocks(nb));
+  }
+#undef FIP_LANES
+  // The words a merged call clears at its start: counts, bboxes and (for the
+  // fused trigger, plain form only: the precision form's compensated
+  // statistics cost the last reprojection more than the separate pass) the
+  // per-region counts.
+  {
+    const bool fuse = im->lanes > 1 && cfg->reproject == 0 && cfg->form == FIP_FORM_PLAIN &&
+                      fip_trigger_fusable(geo);
+    const size_t lanes = (size_t)im->lanes, fc = fuse ? fip_trigger_fuse_counts(geo) : 0;
+    FIP_ALLOC(dalloc(&im->zero_block, lanes * (ntiles + 4) + fc, tot));
+    im->lane_mem.push_back(im->zero_block);
+    im->zero_words = lanes * (ntiles + 4) + fc;
+    for (size_t l = 0; l < lanes; ++l) {
+      im->lane[l].bins.count = im->zero_block + l * ntiles;
+      im->lane[l].bins.bbox = im->zero_block + lanes * ntiles + l * 4;
+    }
+    if (fuse) {
+      im->fuse_count = im->zero_block + lanes * (ntiles + 4);
+      FIP_ALLOC(dalloc(&im->fuse_stats, 3 * (size_t)geo.u * geo.u, tot));
     }
   }
   if (im->custom_fft) {
@@ -567,7 +615,8 @@ int fip_imager_create(fip_imager** out, const fip_imager_config* cfg) {
   // With concurrent lanes a sequence keeps six images, so a lane can start a
   // snapshot while the triggers of the previous ones still read theirs.
   im->ring = im->lanes > 1 ? 6 : 3;
-  for (int k = 0; k < im->ring; ++k) FIP_ALLOC(dalloc(&im->images[k], n2, tot));
+  FIP_ALLOC(dalloc(&im->images[0], im->ring * n2, tot));
+  for (int k = 1; k < im->ring; ++k) im->images[k] = im->images[0] + k * n2;
   FIP_ALLOC(dalloc(&im->maxima, 6, tot));
   FIP_ALLOC(dalloc(&im->result, std::max<size_t>((size_t)geo.u * geo.u, 1), tot));
   FIP_ALLOC(dalloc(&im->d_snap, 3 * 4 * nb, tot));
@@ -578,13 +627,6 @@ int fip_imager_create(fip_imager** out, const fip_imager_config* cfg) {
                            std::max<size_t>((size_t)geo.u * geo.u, 1) * sizeof(float)));
   FIP_ALLOC(dalloc(&im->gather_err, 1, tot));
   FIP_ALLOC(cudaMemset(im->gather_err, 0, sizeof(unsigned)));
-  // Plain form only: the precision form's compensated statistics cost the
-  // last reprojection more than the separate pass (measured 3 % slower).
-  if (im->lanes > 1 && cfg->reproject == 0 && cfg->form == FIP_FORM_PLAIN &&
-      fip_trigger_fusable(geo)) {
-    FIP_ALLOC(dalloc(&im->fuse_count, fip_trigger_fuse_counts(geo), tot));
-    FIP_ALLOC(dalloc(&im->fuse_stats, 3 * (size_t)geo.u * geo.u, tot));
-  }
   FIP_ALLOC(cudaMallocHost((void**)&im->h_err, sizeof(unsigned)));
   *im->h_err = 0;
 
@@ -717,8 +759,13 @@ static int image_snapshot_impl(fip_imager* im, Lane& L, const float* vr, const f
     if (fork) FIP_CUDA(cudaStreamWaitEvent(s, im->ev_join, 0));
     if (targets_ready && targets_ev) FIP_CUDA(cudaStreamWaitEvent(s, targets_ev, 0));
     k = stage_begin(im, ST_REPROJECT, s);
-    FIP_CUDA(fip_launch_reproject_gather(geo, L.pre, L.targets, V, (int)nb, L.bins.bbox + 3,
-                                         image, reinterpret_cast<unsigned*>(image_max),
+    FipGatherBatch in;
+    in.count = 1;
+    in.V[0] = V;
+    in.nb[0] = (int)nb;
+    in.dst[0] = image;
+    in.img_max[0] = reinterpret_cast<unsigned*>(image_max);
+    FIP_CUDA(fip_launch_reproject_gather(geo, in, L.pre, L.targets, L.bins.bbox + 3,
                                          precise ? 1 : 0, s, im->gather_err, fuse));
     stage_end(im, k, s);
     im->launches += 1;
@@ -792,6 +839,101 @@ static int launch_targets_ahead(fip_imager* im, const float* V, cudaEvent_t afte
 static int wait_lane(fip_imager* im, int k, cudaStream_t s) {
   if (im->lanes == 1 || im->timer.on) return FIP_OK;
   FIP_CUDA(cudaStreamWaitEvent(s, im->lane[k % im->lanes].ev_done, 0));
+  return FIP_OK;
+}
+
+// Whether a call's snapshots share launches (image_merged) instead of running
+// on concurrent lanes (kMergedMax).
+static bool merge_ok(const fip_imager* im) {
+  return im->geo.n <= kMergedMax && im->custom_fft && im->lanes > 1 && !im->timer.on &&
+         im->cfg.reproject == 0 && fip_bin_batchable(im->geo);
+}
+
+// Images `count` (<= lanes) snapshots of a call in one launch per stage, on s:
+// snapshot k's visibilities at vr + k * vis_stride (nb[k] of them), its
+// coordinates at B + k * b_stride, its basis at V + 9 k, its image into ring
+// slot slot0 + k.
+static int image_merged(fip_imager* im, int count, const float* vr, const float* vi,
+                        size_t vis_stride, const float* B, size_t b_stride, const float* V,
+                        const size_t* nb, int slot0, cudaStream_t s,
+                        const FipFuse* fuse = nullptr) {
+  const FipGeom& geo = im->geo;
+  for (int k = 0; k < count; ++k) {
+    if (nb[k] > im->cfg.max_baselines)
+      return fail(FIP_ERR_ARG, "nb exceeds the imager's capacity");
+    if (nb[k] == 0) return fail(FIP_ERR_ARG, "nb must be positive");
+  }
+  if (!vr || !vi || !B || !V) return fail(FIP_ERR_ARG, "null device pointer");
+  const bool precise = im->cfg.form == FIP_FORM_PRECISE;
+  const size_t n2 = (size_t)geo.n * geo.n;
+  Lane& L = im->lane[0];
+  FIP_CUDA(cudaMemsetAsync(im->zero_block, 0, im->zero_words * sizeof(unsigned), s));
+  // The pixel mappings need only V: beside everything up to the reprojection
+  // (on s itself, at 512^2, 83 against 76 us a call).
+  if (!precise) {
+    FIP_CUDA(cudaEventRecord(im->ev_fork, s));
+    FIP_CUDA(cudaStreamWaitEvent(im->side, im->ev_fork, 0));
+    FIP_CUDA(fip_launch_targets(geo, V, im->theta_tab, L.targets, im->side, count, n2));
+    FIP_CUDA(cudaEventRecord(im->ev_join, im->side));
+  }
+  FipBinBatch bin;
+  FipGridBatch in{};
+  FipGatherBatch gb;
+  bin.count = in.count = gb.count = count;
+  int vt = FIP_VIS_F32;
+  const bool reduced = precise && im->cfg.vis_storage != FIP_STORE_F32;
+  if (reduced) vt = im->cfg.vis_storage == FIP_STORE_F16 ? FIP_VIS_F16 : FIP_VIS_BF16;
+  bool even = true;
+  for (int k = 0; k < count; ++k) {
+    Lane& K = im->lane[k];
+    float* mx = im->maxima + slot0 + k;
+    bin.s[k] = fip_bin_snap(geo, B + k * b_stride, (int)nb[k], K.bins, K.grid,
+                            reinterpret_cast<unsigned*>(mx));
+    FipGridSnap& g = in.s[k];
+    g.B = B + k * b_stride;
+    g.V = V + 9 * k;
+    g.vr = reduced ? K.q_re : static_cast<const void*>(vr + k * vis_stride);
+    g.vi = reduced ? K.q_im : static_cast<const void*>(vi + k * vis_stride);
+    g.vis_scale = reduced ? K.q_scale : nullptr;
+    g.entries = K.bins.entries;
+    g.work = K.bins.work;
+    g.nwork = K.bins.nwork;
+    g.grid = K.grid;
+    g.scale = geo.cell * (float)(size_t)geo.g;
+    g.g = geo.g;
+    g.hp = geo.hp;
+    g.tiles_c = geo.tiles_c;
+    g.layout = geo.layout;
+    gb.V[k] = V + 9 * k;
+    gb.nb[k] = (int)nb[k];
+    gb.dst[k] = im->images[slot0 + k];
+    gb.img_max[k] = reinterpret_cast<unsigned*>(mx);
+    even = even && nb[k] == nb[0];
+  }
+  // The lanes' list positions together hold ctas * count rows of one launch.
+  FIP_CUDA(fip_launch_bin_batch(bin, L.bins.base, s));
+  if (reduced && even) {
+    FIP_CUDA(fip_launch_quantize(vr, vi, nb[0], vt, L.q_re, L.q_im, L.q_scale, s, count,
+                                 vis_stride, im->cfg.max_baselines));
+    im->launches += 1;
+  } else if (reduced) {
+    for (int k = 0; k < count; ++k) {
+      Lane& K = im->lane[k];
+      FIP_CUDA(fip_launch_quantize(vr + k * vis_stride, vi + k * vis_stride, nb[k], vt, K.q_re,
+                                   K.q_im, K.q_scale, s));
+      im->launches += 1;
+    }
+  }
+  FIP_CUDA(fip_launch_grid_batch(in, vt, grid_compensated(precise, vt), s, im->grid_ctas_per_sm));
+  FIP_CUDA(fip_launch_fft_cols(geo, L.grid, L.bins.bbox, L.colbuf, im->twiddles, im->fft, s, count,
+                               im->grid_stride, im->col_stride));
+  FIP_CUDA(fip_launch_fft_rows(geo, L.colbuf, L.bins.bbox, im->taper, im->twiddles, im->fft,
+                               L.pre, s, count, im->col_stride, n2));
+  if (!precise) FIP_CUDA(cudaStreamWaitEvent(s, im->ev_join, 0));
+  FIP_CUDA(fip_launch_reproject_gather(geo, gb, L.pre, L.targets, L.bins.bbox + 3,
+                                       precise ? 1 : 0, s, im->gather_err, fuse));
+  im->launches += precise ? 7 : 8;  // binning 3, grid, transforms 2, gather (and mapping)
+  im->last_lane = count - 1;
   return FIP_OK;
 }
 
@@ -910,18 +1052,23 @@ int fip_pipe_device(fip_imager* im, const float* vr, const float* vi, const floa
   // (fused into their reprojections when it can be).
   const FipFuse fz = fuse_of(im);
   const bool fused = fuse_ok(im) && result;
-  if (fused) FIP_CUDA(cudaMemsetAsync(im->fuse_count, 0,
-                                      fip_trigger_fuse_counts(im->geo) * sizeof(unsigned), s));
-  FIP_CUDA(cudaEventRecord(im->ev_start, s));
-  const bool ahead = targets_ahead(im);
-  if (ahead) FIP_TRY(launch_targets_ahead(im, V, im->ev_start));
-  for (int k = 0; k < 3; ++k)
-    FIP_TRY(image_on_lane(im, k, vr + (size_t)k * nb, vi + (size_t)k * nb,
-                          B + (size_t)k * nb * 2, V + (size_t)k * 9, nb, im->images[k],
-                          im->maxima + k, s, im->ev_start, ahead, false,
-                          fused ? &fz : nullptr));
-  for (int k = 0; k < 3; ++k) FIP_TRY(wait_lane(im, k, s));
-  im->last_lane = 2 % im->lanes;
+  if (merge_ok(im)) {
+    const size_t nbs[3] = {nb, nb, nb};
+    FIP_TRY(image_merged(im, 3, vr, vi, nb, B, 2 * nb, V, nbs, 0, s, fused ? &fz : nullptr));
+  } else {
+    if (fused) FIP_CUDA(cudaMemsetAsync(im->fuse_count, 0,
+                                        fip_trigger_fuse_counts(im->geo) * sizeof(unsigned), s));
+    FIP_CUDA(cudaEventRecord(im->ev_start, s));
+    const bool ahead = targets_ahead(im);
+    if (ahead) FIP_TRY(launch_targets_ahead(im, V, im->ev_start));
+    for (int k = 0; k < 3; ++k)
+      FIP_TRY(image_on_lane(im, k, vr + (size_t)k * nb, vi + (size_t)k * nb,
+                            B + (size_t)k * nb * 2, V + (size_t)k * 9, nb, im->images[k],
+                            im->maxima + k, s, im->ev_start, ahead, false,
+                            fused ? &fz : nullptr));
+    for (int k = 0; k < 3; ++k) FIP_TRY(wait_lane(im, k, s));
+    im->last_lane = 2 % im->lanes;
+  }
   if (fused) {
     FIP_CUDA(fip_launch_trigger_combine(im->geo, im->fuse_stats, im->maxima, result,
                                         im->cfg.form == FIP_FORM_PRECISE ? 1 : 0, s));
@@ -1254,6 +1401,24 @@ int fip_image_sequence(fip_imager* im, const float* vr, const float* vi, const f
   // recorded on s after that trigger, releases it, so the lanes run up to
   // R - 3 snapshots ahead of the triggers.
   const int R = im->ring;
+  if (merge_ok(im)) {
+    // Groups of three snapshots, alternating between the ring's halves; each
+    // group's triggers (its snapshots with two predecessors) in one launch.
+    for (size_t k = 0; k < nsnap; k += kLanes) {
+      const int count = (int)std::min<size_t>(kLanes, nsnap - k);
+      FIP_TRY(image_merged(im, count, vr + k * nb_stride, vi + k * nb_stride, nb_stride,
+                           B + k * nb_stride * 2, 2 * nb_stride, V + k * 9, nb + k, (int)(k % R),
+                           s));
+      const size_t t0 = k >= 2 ? k - 2 : 0, t1 = k + count >= 2 ? k + count - 2 : 0;
+      if (t1 > t0) {
+        FIP_CUDA(fip_launch_trigger_ring(im->geo, im->images[0], im->maxima, R, (int)(t0 % R),
+                                         (int)(t1 - t0), results + t0 * uu,
+                                         im->cfg.form == FIP_FORM_PRECISE ? 1 : 0, s));
+        im->launches += 1;
+      }
+    }
+    return call_leave(im, s);
+  }
   FIP_CUDA(cudaEventRecord(im->ev_start, s));
   for (size_t k = 0; k < nsnap; ++k) {
     const int slot = (int)(k % R);
@@ -1715,21 +1880,28 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
       if (l.per[c] > 0)
         FIP_CUDA(cudaMemsetAsync(b->seq[c].maxima + 2, 0, l.per[c] * sizeof(float), s));
   }
+  // One reprojection launch per sequence, side by side on the branches.
   FIP_CUDA(cudaEventRecord(b->fork, s));
-  for (int i = 0; i < kBranches; ++i) FIP_CUDA(cudaStreamWaitEvent(b->branch[i], b->fork, 0));
-  for (int k = 0; k < count; ++k) {
-    const BatchSeq& q = b->seq[l.sq[k]];
-    const int j = l.loc[k];
-    cudaStream_t bs = b->branch[k % kBranches];
-    float* img = slots ? slots[k].image : q.images + (j + 2) * q.n2;
-    float* mx = slots ? slots[k].image_max : q.maxima + j + 2;
-    FIP_CUDA(fip_launch_reproject_gather(
-        q.geo, q.pre + j * q.n2, precise ? nullptr : q.targets + j * q.n2, V[k], (int)nb[k],
-        q.bbox + 4 * j + 3, img, reinterpret_cast<unsigned*>(mx), precise ? 1 : 0, bs,
-        b->gather_err));
+  for (int c = 0; c < nseq; ++c) {
+    const BatchSeq& q = b->seq[c];
+    if (l.per[c] == 0) continue;
+    cudaStream_t bs = b->branch[c % kBranches];
+    FIP_CUDA(cudaStreamWaitEvent(bs, b->fork, 0));
+    FipGatherBatch gb;
+    gb.count = l.per[c];
+    for (int k = 0; k < count; ++k) {
+      if (l.sq[k] != c) continue;
+      const int j = l.loc[k];
+      gb.V[j] = V[k];
+      gb.nb[j] = (int)nb[k];
+      gb.dst[j] = slots ? slots[k].image : q.images + (j + 2) * q.n2;
+      gb.img_max[j] = reinterpret_cast<unsigned*>(slots ? slots[k].image_max : q.maxima + j + 2);
+    }
+    FIP_CUDA(fip_launch_reproject_gather(q.geo, gb, q.pre, precise ? nullptr : q.targets,
+                                         q.bbox + 3, precise ? 1 : 0, bs, b->gather_err));
     launches += 1;
   }
-  for (int i = 0; i < kBranches; ++i) {
+  for (int i = 0; i < std::min(nseq, kBranches); ++i) {
     FIP_CUDA(cudaEventRecord(b->join[i], b->branch[i]));
     FIP_CUDA(cudaStreamWaitEvent(s, b->join[i], 0));
   }

@@ -46,7 +46,7 @@ cudaError_t fip_launch_bin(const FipGeom& geo, const float* B, int nb, FipBins& 
 // entry.  base: [fip_bin_ctas(in.count, ...) * in.count][max ntiles] scratch.
 bool fip_bin_batchable(const FipGeom& geo);
 FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBins& bins,
-                        float2* grid);
+                        float2* grid, unsigned* clear = nullptr);
 cudaError_t fip_launch_bin_batch(FipBinBatch& in, unsigned* base, cudaStream_t s);
 // CTAs per snapshot of a binning launch over `count` snapshots of up to
 // nbmax visibilities; ctas * count <= kFipBinCtas.
@@ -89,8 +89,10 @@ cudaError_t fip_launch_correct_c2r(const FipGeom& geo, const float* fft_out, con
 // The reference's pixel mapping of every source pixel -> targets [N*N].
 // theta_tab: the table fip_launch_theta_table fills (bit-identical results,
 // fewer instructions), or null.
+// batch > 1: snapshot k's basis at V + 9 k, its targets at targets + k * stride.
 cudaError_t fip_launch_targets(const FipGeom& geo, const float* V, const float2* theta_tab,
-                               float2* targets, cudaStream_t s);
+                               float2* targets, cudaStream_t s, int batch = 1,
+                               size_t stride = 0);
 // The pixel-mapping kernel's entry (to tell its graph nodes apart).
 const void* fip_targets_kernel();
 // Entries of the theta-terms table of the pixel mapping, and its fill.
@@ -125,10 +127,12 @@ cudaError_t fip_launch_trigger_combine(const FipGeom& geo, const double* stats,
 // err (or null): set to nonzero when a tile lies outside the gather's domain
 // (fip_gather_domain_ok); its image is then not to be trusted.
 // fuse (or null): fuse the call's trigger into this reprojection.
-cudaError_t fip_launch_reproject_gather(const FipGeom& geo, const float* pre,
-                                        const float2* targets, const float* V, int nb,
-                                        const unsigned* pre_max, float* dst, unsigned* img_max,
-                                        int exact_targets, cudaStream_t s, unsigned* err,
+// The snapshots of `in` (one image size), snapshot k's pre, targets and pre_max
+// at base + k * n2 (n2 = N * N; pre_max 4 words apart).
+cudaError_t fip_launch_reproject_gather(const FipGeom& geo, const FipGatherBatch& in,
+                                        const float* pre, const float2* targets,
+                                        const unsigned* pre_max, int exact_targets,
+                                        cudaStream_t s, unsigned* err,
                                         const FipFuse* fuse = nullptr);
 // Whether the plane-to-sky map of basis V (host, row-major 3 x 3) stays in
 // the tile gather's domain over an N x N image: well inside the horizon and
@@ -139,6 +143,11 @@ cudaError_t fip_launch_image_max(const float* img, size_t count, unsigned* out, 
 cudaError_t fip_launch_trigger(const FipGeom& geo, const float* I1, const float* I2,
                                const float* I3, const float* max3, float* stats,
                                float* result, int precise, cudaStream_t s);
+// Triples first .. first + count - 1 of a ring of `ring` images (N * N apart)
+// with maxima[ring]: triple k is images k, k + 1, k + 2 modulo ring.
+cudaError_t fip_launch_trigger_ring(const FipGeom& geo, const float* images, const float* maxima,
+                                    int ring, int first, int count, float* results, int precise,
+                                    cudaStream_t s);
 // Same, the three maxima at separate addresses.
 cudaError_t fip_launch_trigger3(const FipGeom& geo, const float* I1, const float* I2,
                                 const float* I3, const float* m1, const float* m2,
@@ -168,8 +177,11 @@ cudaError_t fip_launch_collapse(const float* v0r, const float* v0i, const float*
 // FP16/BF16 storage of a snapshot's visibilities (one launch): scales
 // receives one power-of-two scale per block of FIP_QBLOCK samples
 // ([fip_qblocks(nb)]), out_re/out_im the values divided by their block's.
+// batch > 1: snapshot k's samples at vr + k * in_stride, its results at
+// out + k * out_stride and scales + k * fip_qblocks(out_stride).
 cudaError_t fip_launch_quantize(const float* vr, const float* vi, size_t nb, int vis_type,
-                                void* out_re, void* out_im, float* scales, cudaStream_t s);
+                                void* out_re, void* out_im, float* scales, cudaStream_t s,
+                                int batch = 1, size_t in_stride = 0, size_t out_stride = 0);
 // The same from raw two-polarisation samples, collapsed to Stokes I on load.
 cudaError_t fip_launch_quantize_raw(const FipRawVis& raw, size_t nb, int vis_type, void* out_re,
                                     void* out_im, float* scales, cudaStream_t s);

@@ -24,11 +24,9 @@
 //     warp-shuffle tile reductions; a batch's sliding window streams each
 //     tile's slices through registers, every image read once for all the
 //     triples it is in.
-#include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -502,6 +500,7 @@ __global__ void __launch_bounds__(kScanThreads) k_bin_scan_tiles(
     carry.z += total.z;
   }
   if (threadIdx.x == 0) {
+    if (sn.clear) *sn.clear = 0;
     sn.offset[ntiles] = carry.x;
     *sn.nwork = min(carry.y, wcap);
     *sn.nmulti = carry.z;
@@ -892,497 +891,6 @@ __global__ void __launch_bounds__(kThreads) k_grid_batch(const __grid_constant__
   }
 }
 
-// Block-wide maximum of non-negative v, folded into *out (float bits) with
-// one atomic per CTA.  All threads of the CTA must call it.
-__device__ __forceinline__ void block_max_to(float v, unsigned* out) {
-  __shared__ float s_m[32];
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) s_m[warp] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float m = 0.f;
-    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) m = fmaxf(m, s_m[w]);
-    atomicMax(out, __float_as_uint(m));
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Band-pruned inverse FFT (power-of-two images), instantiated per
-// M = 2^LM = G / 3 and E = 2^LE values per thread (3 M / E threads).
-// Column pass: P[c][yy] = sum_r1 H[c][r1 mod G] e^{+2 pi i y r1 / G},
-// y = yy - N/2, for the occupied half-plane columns c <= bbox[1] and rows
-// |r1| <= bbox[0].
-// ---------------------------------------------------------------------------
-template <int LM, int LE>
-__host__ __device__ constexpr int fft_threads() { return 3 << (LM - LE); }
-// CTAs per SM the register budget allows: the staged forms hold two
-// buffers of shared memory (two CTAs of 768 or 384 threads); the direct form
-// holds one, so three CTAs of 384 threads fit.
-template <int LM, int LE, bool DIRECT>
-__host__ __device__ constexpr int fft_min_blocks() {
-  return fft_threads<LM, LE>() >= 768 && LE == 4 ? 1 : (DIRECT && LE == 4 ? 3 : 2);
-}
-
-template <int LM, int LE, bool DIRECT>
-__global__ void __launch_bounds__(fft_threads<LM, LE>(), (fft_min_blocks<LM, LE, DIRECT>()))
-    k_fft_cols(const float2* __restrict__ H, const unsigned* __restrict__ bbox,
-               float2* __restrict__ P, const float2* __restrict__ tw, size_t grid_stride,
-               size_t col_stride) {
-  constexpr int M = 1 << LM, g = 3 * M, half = g / 2, n = 2 * M, NT = fft_threads<LM, LE>();
-  extern __shared__ float2 s_fft[];
-  // Batched launches: snapshot blockIdx.y.
-  H += blockIdx.y * grid_stride;
-  P += blockIdx.y * col_stride;
-  bbox += 4 * blockIdx.y;
-  const int k2 = (int)bbox[1];
-  const int k1 = min((int)bbox[0], half);
-  // Row band [lo, hi]; row -G/2 is row +G/2 (counted once).
-  const int lo = (k1 == half) ? 1 - k1 : -k1, hi = k1;
-  // Stage the band densely (coalesced): st[r - lo] = H[c][r mod G]; or
-  // (DIRECT) read it from global memory in the first pass.
-  // A band no wider than M is staged pre-twiddled for the three
-  // sub-transforms (fipfft::stage_pre).
-  float2* st = s_fft + fipfft::stage_offset(g);
-  const bool fold = !DIRECT && hi - lo + 1 <= M;
-  auto band = [&](int c, int r) -> float2 { return H[(size_t)c * g + (r < 0 ? r + g : r)]; };
-  // The staged form is persistent over columns (blockIdx.x + k gridDim.x):
-  // a thread's first staged element of the next column is loaded while the
-  // current column is transformed.
-  const int r0 = lo + (int)threadIdx.x;
-  float2 pf = make_float2(0.f, 0.f);
-  if (!DIRECT && (int)blockIdx.x <= k2 && r0 <= hi) pf = band(blockIdx.x, r0);
-  for (int c = blockIdx.x; c <= k2; c += gridDim.x) {
-    // Pass twiddles (registers): loaded after the staging loop, so their
-    // latency overlaps the staging barrier without holding registers through
-    // the loop (measured faster here than loading them up front).
-    fipfft::PassTw<LM, LE> pt;
-    if (DIRECT) pt.load(tw + g, fipfft::sub_lane<LM, LE>(threadIdx.x));
-    if (fold) {
-      fipfft::StageTw w(tw, g, r0, NT);
-      if (r0 <= hi) fipfft::stage_pre<M>(st, r0, pf, w.w1, w.w2);
-      w.next();
-      for (int i = threadIdx.x + NT; i <= hi - lo; i += NT, w.next()) {
-        const int r = i + lo;
-        fipfft::stage_pre<M>(st, r, band(c, r), w.w1, w.w2);
-      }
-    } else if (!DIRECT) {
-      if (r0 <= hi) st[threadIdx.x] = pf;
-      for (int i = threadIdx.x + NT; i <= hi - lo; i += NT) st[i] = band(c, i + lo);
-    }
-    if (!DIRECT) {
-      pt.load(tw + g, fipfft::sub_lane<LM, LE>(threadIdx.x));
-      if (fold) fipfft::zero_pre<M>(st, lo, hi, threadIdx.x, NT);
-      __syncthreads();
-      // The next column's first element, in flight during this transform.
-      const int nx = c + gridDim.x;
-      if (nx <= k2 && r0 <= hi) pf = band(nx, r0);
-    }
-    if (fold) {
-      fipfft::run_pre<LM, LE>(s_fft, pt);
-    } else {
-      auto load = [&](int r) -> float2 { return DIRECT ? band(c, r) : st[r - lo]; };
-      fipfft::run<LM, LE, DIRECT>(s_fft, tw, pt, lo, hi, load);
-    }
-    float4* out = reinterpret_cast<float4*>(P + (size_t)c * n);
-    for (int o2 = threadIdx.x; o2 < n / 2; o2 += NT) {
-      float2 ab[2];
-      fipfft::fetch_run<LM, LE, 2, DIRECT>(s_fft, 2 * o2, ab);
-      out[o2] = make_float4(ab[0].x, ab[0].y, ab[1].x, ab[1].y);
-    }
-    // The next staging writes the second buffer: when the last pass left
-    // its outputs there, every thread must be done reading them.
-    if constexpr (!DIRECT && ((fipfft::pass_count<LM, LE>() - 1) & 1)) __syncthreads();
-  }
-}
-
-// Bulk tensor copies (TMA) with an mbarrier, for the row pass's band copy.
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-// Bounded wait for phase `parity` of *bar: false if it did not complete
-// within kMbarSpin polls.
-constexpr unsigned kMbarSpin = 1u << 20;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  const unsigned a = smem_u32(bar);
-  for (unsigned it = 0; it < kMbarSpin; ++it) {
-    unsigned done = 0;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y,
-                                            int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
-// The row pass's band copy: columns 0 .. K2 (at most kBandCap; wider bands
-// read global memory) of a row pair, kBandBox columns per bulk copy, 16
-// bytes (rows yy1, yy1 + 1 of one column) each.
-constexpr int kBandCap = 1024;
-constexpr int kBandBox = 256;
-// The copy's buffer follows the direct form's pass buffer; a bulk tensor
-// copy's shared-memory destination must be 128-byte aligned, and dynamic
-// shared memory starts after the kernel's static shared memory (not on a
-// 128-byte boundary), so the buffer is aligned at run time within 128 bytes
-// of slack.
-template <int LM>
-__host__ __device__ constexpr size_t band_offset() {  // bytes
-  return (size_t)fipfft::direct_smem_elems(3 << LM) * sizeof(float2);
-}
-template <int LM>
-__host__ __device__ constexpr size_t band_smem_bytes() {
-  return band_offset<LM>() + 128 + (size_t)kBandCap * 16;
-}
-
-// Row pass for image rows yy1 = 2b, yy2 = 2b+1: their Hermitian spectra
-// X1, X2 (the column-pass output, extended by X(-c) = conj X(c)) are packed as
-// Z = X1 + i X2 so one complex transform yields both real rows.  The epilogue
-// is the reference's crop/correction (FIPkernels.cu:256-287): the image pixel
-// is |out| / (taper|x| taper|y| norm^2) (the checkerboard signs cancel
-// against the centred grid origin), applied as a product of the reciprocal
-// table rck[t] = 1 / (taper[t] norm).
-// BAND (with DIRECT, persistent over row pairs): the first pass reads the
-// row pair's band from a shared-memory copy that bulk tensor copies bring in
-// one row pair ahead (band_map: the column-pass output as floats [batch][G/2
-// + 1][2 N]); a copy that does not arrive within the wait limit switches the
-// CTA to global reads (same results).
-template <int LM, int LE, bool DIRECT, bool BAND = false>
-__global__ void __launch_bounds__(fft_threads<LM, LE>(), (fft_min_blocks<LM, LE, DIRECT>()))
-    k_fft_rows(const float2* __restrict__ P, unsigned* bbox,
-               const float* __restrict__ rck, float* __restrict__ pre,
-               const float2* __restrict__ tw, size_t col_stride, size_t pre_stride,
-               const __grid_constant__ CUtensorMap band_map) {
-  static_assert(!BAND || DIRECT, "the band copy replaces the direct form's global reads");
-  constexpr int M = 1 << LM, g = 3 * M, half = g / 2, n = 2 * M, h = M, NT = fft_threads<LM, LE>();
-  extern __shared__ float2 s_fft[];
-  // Batched launches: snapshot blockIdx.y.
-  P += blockIdx.y * col_stride;
-  pre += blockIdx.y * pre_stride;
-  bbox += 4 * blockIdx.y;
-  const int k2 = min((int)bbox[1], half);
-  // Column band [lo, hi]; column -G/2 is column +G/2 (counted once).
-  const int lo = (k2 == half) ? 1 - k2 : -k2, hi = k2;
-  // Stage Z[c] = X1[c] + i X2[c] at st[c - lo], with X(-c) = conj X(c):
-  // one 16-byte load per occupied column c (the column pass stores
-  // P[c][yy]), written at c and -c.
-  float2* st = s_fft + fipfft::stage_offset(g);
-  // Pass twiddles first: their loads overlap the staging loads.
-  fipfft::PassTw<LM, LE> pt;
-  pt.load(tw + g, fipfft::sub_lane<LM, LE>(threadIdx.x));
-  // A band no wider than M is staged pre-twiddled (fipfft::stage_pre).
-  const bool fold = !DIRECT && hi - lo + 1 <= M;
-  // The staged form is persistent over row pairs (blockIdx.x + k gridDim.x):
-  // a thread's first staged column of the next row pair is loaded into
-  // registers while the current pair is transformed, so its latency leaves
-  // the staging step (two columns measured slower: more spills).
-  constexpr int kPf = 1;
-  float4 pf[kPf];
-  auto col_load = [&](int c, int yy) -> float4 {
-    return *reinterpret_cast<const float4*>(P + (size_t)c * n + yy);
-  };
-#pragma unroll
-  for (int m = 0; m < kPf; ++m) {
-    const int c = threadIdx.x + m * NT;
-    if (!DIRECT && c <= k2) pf[m] = col_load(c, 2 * blockIdx.x);
-  }
-  // BAND: the copy's buffer, its mbarrier, and the parity of a copy issued
-  // but not yet consumed (-1: none).
-  char* band_raw = reinterpret_cast<char*>(s_fft) + band_offset<LM>();
-  float4* sband =
-      reinterpret_cast<float4*>(band_raw + ((128u - (smem_u32(band_raw) & 127u)) & 127u));
-  __shared__ uint64_t s_bandbar;
-  // Uniform over the CTA; a misaligned buffer (not expected) reads global
-  // memory instead.
-  bool band = BAND && k2 + 1 <= kBandCap && (smem_u32(sband) & 127u) == 0;
-  int pend = -1;
-  const int nbox = (k2 + kBandBox) / kBandBox;  // boxes covering columns 0 .. k2
-  auto issue = [&](int rpair) {  // one thread
-    mbar_expect_tx(&s_bandbar, (unsigned)(nbox * kBandBox * 16));
-    for (int b = 0; b < nbox; ++b)
-      tma_load_3d(sband + b * kBandBox, &band_map, 4 * rpair, b * kBandBox, (int)blockIdx.y,
-                  &s_bandbar);
-  };
-  if (BAND && band) {
-    if (threadIdx.x == 0) {
-      mbar_init(&s_bandbar, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    __syncthreads();
-    if (blockIdx.x < n / 2) {
-      if (threadIdx.x == 0) issue(blockIdx.x);
-      pend = 0;
-    }
-  }
-  float vmax = 0.f;
-  int it = 0;
-  for (int rp = blockIdx.x; rp < n / 2; rp += gridDim.x, ++it) {
-    const int yy1 = 2 * rp;
-    if (BAND && band) {
-      const bool got = mbar_wait(&s_bandbar, (unsigned)(it & 1));
-      band = __syncthreads_and(got) != 0;
-      if (band) pend = -1;  // else the copy stays pending: drained at the end
-    }
-    if (!DIRECT) {
-      fipfft::StageTw w(tw, g, threadIdx.x, NT);
-      auto stage = [&](int c, const float4& ab) {
-        float ay = ab.y, by = ab.w;
-        if (c == 0 || c == half) {  // self-conjugate bins are real
-          ay = 0.f;
-          by = 0.f;
-        }
-        const float2 zp = make_float2(ab.x - by, ay + ab.z);
-        const float2 zm = make_float2(ab.x + by, ab.z - ay);  // conj X1 + i conj X2
-        if (fold) {
-          // w^{-c} = conj w^c
-          fipfft::stage_pre<M>(st, c, zp, w.w1, w.w2);
-          if (c > 0 && -c >= lo)
-            fipfft::stage_pre<M>(st, -c, zm, make_float2(w.w1.x, -w.w1.y),
-                                 make_float2(w.w2.x, -w.w2.y));
-        } else {
-          st[c - lo] = zp;
-          if (c > 0 && -c >= lo) st[-c - lo] = zm;
-        }
-      };
-#pragma unroll
-      for (int m = 0; m < kPf; ++m, w.next()) {
-        const int c = threadIdx.x + m * NT;
-        if (c <= k2) stage(c, pf[m]);
-      }
-      for (int c = threadIdx.x + kPf * NT; c <= k2; c += NT, w.next()) stage(c, col_load(c, yy1));
-      if (fold) fipfft::zero_pre<M>(st, lo, hi, threadIdx.x, NT);
-      __syncthreads();
-      // The next row pair's first columns, in flight during this transform.
-      const int nx = rp + gridDim.x;
-#pragma unroll
-      for (int m = 0; m < kPf; ++m) {
-        const int c = threadIdx.x + m * NT;
-        if (nx < n / 2 && c <= k2) pf[m] = col_load(c, 2 * nx);
-      }
-    }
-    // DIRECT: Z[c] straight from the column-pass output (L2-resident).
-    auto zval = [&](int c) -> float2 {
-      const int a = c < 0 ? -c : c;
-      const float4 ab = (BAND && band) ? sband[a] : col_load(a, yy1);
-      float ay = ab.y, by = ab.w;
-      if (a == 0 || a == half) {
-        ay = 0.f;
-        by = 0.f;
-      }
-      return c >= 0 ? make_float2(ab.x - by, ay + ab.z) : make_float2(ab.x + by, ab.z - ay);
-    };
-    auto load = [&](int c) -> float2 { return DIRECT ? zval(c) : st[c - lo]; };
-    if (fold) {
-      fipfft::run_pre<LM, LE>(s_fft, pt);
-    } else if constexpr (BAND) {
-      // Once every thread holds its band values, the next row pair's copy
-      // goes into the buffer (it lands during this pair's passes).
-      auto loaded = [&]() {
-        if (!band) return;
-        __syncthreads();
-        const int nx = rp + (int)gridDim.x;
-        if (nx < n / 2) {
-          if (threadIdx.x == 0) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            issue(nx);
-          }
-          pend = (it + 1) & 1;
-        }
-      };
-      fipfft::run<LM, LE, DIRECT>(s_fft, tw, pt, lo, hi, load, loaded);
-    } else {
-      fipfft::run<LM, LE, DIRECT>(s_fft, tw, pt, lo, hi, load);
-    }
-    const float ry1 = rck[abs(yy1 - h)], ry2 = rck[abs(yy1 + 1 - h)];
-    float4* row1 = reinterpret_cast<float4*>(pre + (size_t)yy1 * n);
-    float4* row2 = reinterpret_cast<float4*>(pre + (size_t)(yy1 + 1) * n);
-    // The epilogue's correction factors, all loads issued before the first
-    // output is formed.
-    constexpr int KQ = (n / 4 + NT - 1) / NT;
-    float rxs[KQ][4];
-#pragma unroll
-    for (int q = 0; q < KQ; ++q) {
-      const int o4 = threadIdx.x + q * NT;
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        rxs[q][e] = o4 < n / 4 ? __ldg(&rck[abs(4 * o4 + e - h)]) : 0.f;
-    }
-#pragma unroll
-    for (int q = 0; q < KQ; ++q) {
-      const int o4 = threadIdx.x + q * NT;
-      if (o4 < n / 4) {
-        float a[4], b[4];
-        float2 v[4];
-        fipfft::fetch_run<LM, LE, 4, DIRECT>(s_fft, 4 * o4, v);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float rx = rxs[q][e];
-          a[e] = fabsf(v[e].x * (rx * ry1));
-          b[e] = fabsf(v[e].y * (rx * ry2));
-          vmax = fmaxf(vmax, fmaxf(a[e], b[e]));
-        }
-        row1[o4] = make_float4(a[0], a[1], a[2], a[3]);
-        row2[o4] = make_float4(b[0], b[1], b[2], b[3]);
-      }
-    }
-    // The next staging writes the second buffer: when the last pass left
-    // its outputs there, every thread must be done reading them.
-    if constexpr (!DIRECT && ((fipfft::pass_count<LM, LE>() - 1) & 1)) __syncthreads();
-  }
-  // A copy still pending (its wait ran out) lands before the CTA's shared
-  // memory goes away (bounded, like every wait here).
-  if (BAND && pend >= 0 && threadIdx.x == 0) mbar_wait(&s_bandbar, (unsigned)pend);
-  // Image maximum (bbox[3], float bits; zeroed by the binning), which
-  // scales the reprojection's fixed-point sums.
-  block_max_to(vmax, &bbox[3]);
-}
-
-// Split forms of the two passes: one CTA of M / E threads per (column or row
-// pair, sub-transform s), grid.y = s, grid.z = snapshot of a batch.  Three
-// times the CTAs of a quarter of the size: each CTA's barriers hold four
-// warps instead of twelve, and CTAs at different phases share an SM.  Each
-// CTA stages the band itself (in its second buffer when it fits, else reads
-// it from global memory) and writes its outputs X[3 q + s] directly.
-template <int LM, int LE>
-__host__ __device__ constexpr int split_threads() { return 1 << (LM - LE); }
-
-template <int LM, int LE>
-__global__ void __launch_bounds__(split_threads<LM, LE>(), (LE == 4 ? 6 : 4))
-    k_fft_cols_split(const float2* __restrict__ H, const unsigned* __restrict__ bbox,
-                     float2* __restrict__ P, const float2* __restrict__ tw, size_t grid_stride,
-                     size_t col_stride) {
-  constexpr int M = 1 << LM, g = 3 * M, half = g / 2, n = 2 * M, NT = split_threads<LM, LE>();
-  constexpr int kCap = fipfft::sub_stride(M);  // staging capacity (the second buffer)
-  extern __shared__ float2 s_fft[];
-  H += blockIdx.z * grid_stride;
-  P += blockIdx.z * col_stride;
-  bbox += 4 * blockIdx.z;
-  const int c = blockIdx.x, s = blockIdx.y;
-  const int k2 = (int)bbox[1];
-  if (c > k2) return;
-  const int k1 = min((int)bbox[0], half);
-  const int lo = (k1 == half) ? 1 - k1 : -k1, hi = k1;
-  const float2* col = H + (size_t)c * g;
-  float2* st = s_fft + kCap;
-  const bool staged = hi - lo + 1 <= kCap;
-  if (staged)
-    for (int i = threadIdx.x; i <= hi - lo; i += NT) {
-      const int r = i + lo;
-      st[i] = col[r < 0 ? r + g : r];
-    }
-  __syncthreads();
-  auto load = [&](int r) -> float2 { return staged ? st[r - lo] : col[r < 0 ? r + g : r]; };
-  fipfft::PassTw<LM, LE> pt;
-  pt.load(tw + g, threadIdx.x);
-  fipfft::run_single<LM, LE>(s_fft, s, tw, pt, lo, hi, load);
-  float2* out = P + (size_t)c * n;
-  for (int q = threadIdx.x; q < M; q += NT) {
-    const int pp = 3 * q + s;  // output p = pp (mod G), kept when |p| <= M
-    const int o = pp < M ? pp + M : (pp >= 2 * M ? pp - 2 * M : -1);
-    if (o >= 0) out[o] = fipfft::single_out<LM, LE>(s_fft, q);
-  }
-}
-
-template <int LM, int LE>
-__global__ void __launch_bounds__(split_threads<LM, LE>(), (LE == 4 ? 6 : 4))
-    k_fft_rows_split(const float2* __restrict__ P, unsigned* bbox, const float* __restrict__ rck,
-                     float* __restrict__ pre, const float2* __restrict__ tw, size_t col_stride,
-                     size_t pre_stride) {
-  constexpr int M = 1 << LM, g = 3 * M, half = g / 2, n = 2 * M, h = M;
-  constexpr int NT = split_threads<LM, LE>(), kCap = fipfft::sub_stride(M);
-  extern __shared__ float2 s_fft[];
-  P += blockIdx.z * col_stride;
-  pre += blockIdx.z * pre_stride;
-  bbox += 4 * blockIdx.z;
-  const int yy1 = 2 * blockIdx.x, s = blockIdx.y;
-  const int k2 = min((int)bbox[1], half);
-  const int lo = (k2 == half) ? 1 - k2 : -k2, hi = k2;
-  // Z[c] = X1[c] + i X2[c], X(-c) = conj X(c), from the column-pass output.
-  auto zval = [&](int c) -> float2 {
-    const int a = c < 0 ? -c : c;
-    const float4 ab = *reinterpret_cast<const float4*>(P + (size_t)a * n + yy1);
-    float ay = ab.y, by = ab.w;
-    if (a == 0 || a == half) {  // self-conjugate bins are real
-      ay = 0.f;
-      by = 0.f;
-    }
-    return c >= 0 ? make_float2(ab.x - by, ay + ab.z) : make_float2(ab.x + by, ab.z - ay);
-  };
-  float2* st = s_fft + kCap;
-  const bool staged = hi - lo + 1 <= kCap;
-  if (staged)
-    for (int c = threadIdx.x; c <= k2; c += NT) {
-      const float4 ab = *reinterpret_cast<const float4*>(P + (size_t)c * n + yy1);
-      float ay = ab.y, by = ab.w;
-      if (c == 0 || c == half) {
-        ay = 0.f;
-        by = 0.f;
-      }
-      st[c - lo] = make_float2(ab.x - by, ay + ab.z);
-      if (c > 0 && -c >= lo) st[-c - lo] = make_float2(ab.x + by, ab.z - ay);
-    }
-  __syncthreads();
-  auto load = [&](int c) -> float2 { return staged ? st[c - lo] : zval(c); };
-  fipfft::PassTw<LM, LE> pt;
-  pt.load(tw + g, threadIdx.x);
-  fipfft::run_single<LM, LE>(s_fft, s, tw, pt, lo, hi, load);
-  const float ry1 = rck[abs(yy1 - h)], ry2 = rck[abs(yy1 + 1 - h)];
-  float* row1 = pre + (size_t)yy1 * n;
-  float* row2 = row1 + n;
-  float vmax = 0.f;
-  for (int q = threadIdx.x; q < M; q += NT) {
-    const int pp = 3 * q + s;
-    const int o = pp < M ? pp + M : (pp >= 2 * M ? pp - 2 * M : -1);
-    if (o >= 0) {
-      const float2 v = fipfft::single_out<LM, LE>(s_fft, q);
-      const float rx = rck[abs(o - h)];
-      const float a = fabsf(v.x * (rx * ry1)), b = fabsf(v.y * (rx * ry2));
-      row1[o] = a;
-      row2[o] = b;
-      vmax = fmaxf(vmax, fmaxf(a, b));
-    }
-  }
-  block_max_to(vmax, &bbox[3]);
-}
-
-// Crop + correction of the cuFFT C2R output (images whose grid side is not
-// 3 * 2^k): row (y mod G), column (x mod G), row stride G + 2 floats.
-__global__ void k_correct_c2r(const float* __restrict__ fft_out, const float* __restrict__ ck,
-                              int n, int g, float* __restrict__ pre, unsigned* pre_max) {
-  const int xx = blockIdx.x * blockDim.x + threadIdx.x, yy = blockIdx.y;
-  float v = 0.f;
-  if (xx < n) {
-    const int h = n / 2;
-    const long x = (long)xx - h, y = (long)yy - h;
-    const int row = (int)(y < 0 ? y + g : y), col = (int)(x < 0 ? x + g : x);
-    float px = fft_out[(size_t)row * (size_t)(g + 2) + col];
-    const float norm = FIP_CONV_NORM;
-    px *= 1 / (ck[labs(x)] * ck[labs(y)] * norm * norm);
-    v = fabs(px);
-    pre[(size_t)yy * n + xx] = v;
-  }
-  block_max_to(v, pre_max);
-}
-
 // ---------------------------------------------------------------------------
 // Reprojection (FIPkernels.cu:289-413).
 // ---------------------------------------------------------------------------
@@ -1392,8 +900,15 @@ __global__ void k_correct_c2r(const float* __restrict__ fft_out, const float* __
 // gridding and the FFT on a side stream.
 constexpr int kTargetsPerThread = 4;
 // ttab: the theta-terms table (fipref::kThetaTabSize entries) or null.
+// MANY: launches over several snapshots (blockIdx.z).
+template <bool MANY>
 __global__ void k_targets(const float* __restrict__ V, int n, float dc,
-                          const float2* __restrict__ ttab, float2* __restrict__ tg) {
+                          const float2* __restrict__ ttab, float2* __restrict__ tg,
+                          size_t stride) {
+  if (MANY) {
+    V += 9 * blockIdx.z;
+    tg += blockIdx.z * stride;
+  }
   const int j = blockIdx.y;
   const fipref::Frame fr{V[0], V[1], V[3], V[4], V[8], V[6], V[7], dc};
 #pragma unroll
@@ -1741,11 +1256,22 @@ constexpr int kSeg = 2;
 constexpr int kPoly = 4 * kSeg;
 static_assert(kPoly <= 32 && (kPoly & (kPoly - 1)) == 0, "one warp's lanes, a power of two");
 
-template <bool EXACT>
+// MANY: a launch over several snapshots (blockIdx.y); launches of one keep
+// every pointer in the constant bank (with MANY's register pairs for the
+// per-snapshot pointers the splats spill more: a 4096^2 plain call 969
+// against 949 us).
+template <bool EXACT, bool MANY>
 __global__ void __launch_bounds__(kThreads, EXACT ? 5 : 8) k_reproject_gather(
-    const float* __restrict__ pre, const float2* __restrict__ tg, const float* __restrict__ V,
-    int n, int nb, float cell, float delta, const unsigned* __restrict__ pre_max,
-    float* __restrict__ dst, unsigned* img_max, unsigned* err, const FipTriggerFuse fuse) {
+    const __grid_constant__ FipGatherBatch in, const float* __restrict__ pre,
+    const float2* __restrict__ tg, int n, float cell, float delta,
+    const unsigned* __restrict__ pre_max, unsigned* err,
+    const __grid_constant__ FipTriggerFuse fuse) {
+  const int snap = MANY ? (int)blockIdx.y : 0;
+  const float* __restrict__ V = in.V[snap];
+  if (MANY) {
+    pre += snap * (size_t)n * n;
+    if (!EXACT) tg += snap * (size_t)n * n;
+  }
   __shared__ __align__(16) unsigned s_tile[kTW * kTR];
   __shared__ int s_base[kMaxRows];  // pixel index of row r's first candidate minus its number
   __shared__ int s_off[kMaxRows + 1];
@@ -1838,7 +1364,6 @@ __global__ void __launch_bounds__(kThreads, EXACT ? 5 : 8) k_reproject_gather(
   const float sag = s_sag + 1e-3f;
   const int jlo = (int)fmaxf(0.f, ceilf(fmaxf(bmin + h - sag, -1.f)));
   const int jhi = (int)fminf((float)(n - 1), floorf(fminf(bmax + h + sag, (float)n)));
-  const float inv_nb = 1.0f / static_cast<float>(nb);
   const size_t half = n / 2;
   const float lim = half - 1;  // the reference compares |LL| with size_t (N/2 - 1)
   // A candidate that reaches the tile has LL in [c0 - h - 1, c0 - h + kDT)
@@ -1859,9 +1384,8 @@ __global__ void __launch_bounds__(kThreads, EXACT ? 5 : 8) k_reproject_gather(
   const float parea = s_parea;  // preimage polygon's area (shoelace)
   int sh = 0;
   while (sh < 12 && parea > (float)(2 * kDT * kDT) * (float)(1 << sh)) ++sh;
-  const float pmax = __uint_as_float(*pre_max);
+  const float pmax = __uint_as_float(pre_max[4 * snap]);
   const float qk = pmax > 0.f ? 268435456.0f / (pmax * (float)(1 << sh)) : 0.f;
-  const float deq = pmax * inv_nb * ((float)(1 << sh) / 268435456.0f);
   // Precision form: the tile's constants, from FP64 by a thread of the last
   // warp (idle in the row-interval step unless a chunk has 256 rows); every
   // thread reads them after the chunk's barriers, before its first splat.
@@ -2000,6 +1524,13 @@ __global__ void __launch_bounds__(kThreads, EXACT ? 5 : 8) k_reproject_gather(
     }
     __syncthreads();  // the next chunk rewrites the row offsets
   }
+  // (Per-snapshot values are read from the parameters only here, so that none
+  // of them holds a register through the splats.)
+  const float deq = __uint_as_float(pre_max[4 * snap]) *
+                    (1.0f / static_cast<float>(in.nb[snap])) *
+                    ((float)(1 << sh) / 268435456.0f);
+  float* __restrict__ dst = in.dst[snap];
+  unsigned* img_max = in.img_max[snap];
   float vmax = 0.f;
   for (int k = threadIdx.x; k < kDT * kDT / 4; k += kThreads) {
     const int lr = (4 * k) / kDT, g4 = ((4 * k) % kDT) >> 2;
@@ -2103,7 +1634,8 @@ __global__ void k_image_max(const float* __restrict__ img, size_t count, unsigne
 // M = max(0, max D), R = sum min(D/I2c, 1) (NaN counts 1).
 // PRECISE: Neumaier-compensated S and R, FP64 combine.
 // ---------------------------------------------------------------------------
-template <bool PRECISE>
+// RING: the triples of a ring of images (fip_launch_trigger_ring).
+template <bool PRECISE, bool RING>
 __global__ void __launch_bounds__(kThreads) k_trigger(const float* __restrict__ I1,
                                                       const float* __restrict__ I2,
                                                       const float* __restrict__ I3,
@@ -2112,13 +1644,30 @@ __global__ void __launch_bounds__(kThreads) k_trigger(const float* __restrict__ 
                                                       const float* __restrict__ m3, int n,
                                                       int t, int u, int vec,
                                                       float* __restrict__ result,
-                                                      size_t img_stride, size_t res_stride) {
-  // Batched launches: triple blockIdx.y is images y, y+1, y+2 of a linear ring
-  // (stride img_stride) with maxima m1[y], m2[y], m3[y].
-  I1 += blockIdx.y * img_stride;
-  I2 += blockIdx.y * img_stride;
-  I3 += blockIdx.y * img_stride;
-  const float max3[3] = {m1[blockIdx.y], m2[blockIdx.y], m3[blockIdx.y]};
+                                                      size_t img_stride, size_t res_stride,
+                                                      int ring, int first) {
+  float max3[3];
+  if (RING) {
+    // Triple blockIdx.y is images k, k + 1, k + 2 (k = first + y, modulo
+    // ring) of the ring at I1 with maxima m1[ring].
+    const float* base = I1;
+    const int k0 = (first + (int)blockIdx.y) % ring, k1 = (k0 + 1) % ring, k2 = (k0 + 2) % ring;
+    I1 = base + k0 * img_stride;
+    I2 = base + k1 * img_stride;
+    I3 = base + k2 * img_stride;
+    max3[0] = m1[k0];
+    max3[1] = m1[k1];
+    max3[2] = m1[k2];
+  } else {
+    // Batched launches: triple blockIdx.y is images y, y+1, y+2 of a linear
+    // ring (stride img_stride) with maxima m1[y], m2[y], m3[y].
+    I1 += blockIdx.y * img_stride;
+    I2 += blockIdx.y * img_stride;
+    I3 += blockIdx.y * img_stride;
+    max3[0] = m1[blockIdx.y];
+    max3[1] = m2[blockIdx.y];
+    max3[2] = m3[blockIdx.y];
+  }
   result += blockIdx.y * res_stride;
   const int lane = threadIdx.x & 31;
   const int b = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -2227,32 +1776,6 @@ inline int sm_count() {
 // Launchers
 // ---------------------------------------------------------------------------
 
-bool fip_fft_plan(int g, fipfft::Plan& p, int values_per_thread) {
-  if (g < 48 || g % 3 != 0) return false;
-  const int m = g / 3;
-  if (m & (m - 1)) return false;
-  int lm = 0;
-  while ((1 << lm) < m) ++lm;
-  // Instantiated: 8 values per thread for M = 2^4..2^11, 16 for 2^5..2^12
-  // (<= 768 threads).  Default: 8 up to M = 1024 (N = 2048), 16 beyond -- at
-  // M = 2048 the 16-value row pass takes about two thirds of the 8-value one's
-  // time on B200, and the autotuner picks it there.
-  int le = (lm <= 10) ? 3 : 4;
-  if (values_per_thread == 8) le = 3;
-  if (values_per_thread == 16) le = 4;
-  if (le == 3 && (lm < 4 || lm > 11)) return false;
-  if (le == 4 && (lm < 5 || lm > 12)) return false;
-  p.g = g;
-  p.m = m;
-  p.lm = lm;
-  p.le = le;
-  p.e = 1 << le;
-  p.nt = 3 * (m >> le);
-  p.split = 0;
-  p.direct = 0;
-  return true;
-}
-
 cudaError_t fip_launch_taper(float* taper, const FipGeom& geo, cudaStream_t s) {
   const int cnt = geo.n / 2 + 1;
   k_taper<<<(cnt + kThreads - 1) / kThreads, kThreads, 0, s>>>(taper, (size_t)geo.n,
@@ -2273,7 +1796,7 @@ int fip_bin_ctas(int count, size_t nbmax) {
 }
 
 FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBins& bins,
-                        float2* grid) {
+                        float2* grid, unsigned* clear) {
   FipBinSnap q{};
   q.B = B;
   q.nb = nb;
@@ -2294,6 +1817,7 @@ FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBin
   q.multi = bins.multi;
   q.nmulti = bins.nmulti;
   q.grid = grid;
+  q.clear = clear;
   return q;
 }
 
@@ -2406,219 +1930,15 @@ cudaError_t fip_launch_grid_batch(const FipGridBatch& in, int vis_type, int comp
   return cudaGetLastError();
 }
 
-// The transforms' dynamic shared memory depends on the grid side.  Their
-// limit is raised to the most the device allows next to the kernel's static
-// shared memory, the same value for every caller, so imagers of different
-// sizes launching from concurrent host threads never lower it under one
-// another's launch.
-static cudaError_t fft_smem_attr(const void* fn, size_t smem) {
-  int dev = 0, optin = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess)
-    e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess) return e;
-  cudaFuncAttributes fa{};
-  e = cudaFuncGetAttributes(&fa, fn);
-  if (e != cudaSuccess) return e;
-  const int most = optin - (int)fa.sharedSizeBytes;  // static + dynamic <= opt-in maximum
-  if (smem > (size_t)most) return cudaErrorInvalidConfiguration;
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-}
-
-template <int LM, int LE>
-static cudaError_t launch_cols(const FipGeom& geo, const float2* grid, const unsigned* bbox,
-                               float2* colbuf, const float2* tw, cudaStream_t s, int batch,
-                               size_t grid_stride, size_t col_stride, int split, int direct) {
-  size_t smem;
-  cudaError_t e;
-  if (split) {
-    smem = 2 * (size_t)fipfft::sub_stride(1 << LM) * sizeof(float2);
-    if ((e = fft_smem_attr((const void*)k_fft_cols_split<LM, LE>, smem)) != cudaSuccess)
-      return e;
-    k_fft_cols_split<LM, LE><<<dim3(geo.hp, 3, batch), split_threads<LM, LE>(), smem, s>>>(
-        grid, bbox, colbuf, tw, grid_stride, col_stride);
-    return cudaGetLastError();
-  }
-  if (direct == 1) {  // (2: the row pass's band copy; the column pass stays staged)
-    smem = (size_t)fipfft::direct_smem_elems(geo.g) * sizeof(float2);
-    e = fft_smem_attr((const void*)k_fft_cols<LM, LE, true>, smem);
-    if (e != cudaSuccess) return e;
-    k_fft_cols<LM, LE, true><<<dim3(geo.hp, batch), fft_threads<LM, LE>(), smem, s>>>(
-        grid, bbox, colbuf, tw, grid_stride, col_stride);
-    return cudaGetLastError();
-  }
-  smem = (size_t)fipfft::smem_elems(geo.g) * sizeof(float2);
-  e = fft_smem_attr((const void*)k_fft_cols<LM, LE, false>, smem);
-  if (e != cudaSuccess) return e;
-  // Persistent over columns: the CTAs that fit at once.
-  // (Queried once per instantiation: the shape and shared memory are fixed by it.)
-  static const int per_sm = [&] {
-    int v = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_fft_cols<LM, LE, false>,
-                                                      fft_threads<LM, LE>(), smem) != cudaSuccess)
-      v = 1;
-    return std::max(v, 1);
-  }();
-  const int ctas = std::max(1, std::min(geo.hp, per_sm * sm_count()));
-  k_fft_cols<LM, LE, false><<<dim3(ctas, batch), fft_threads<LM, LE>(), smem, s>>>(
-      grid, bbox, colbuf, tw, grid_stride, col_stride);
-  return cudaGetLastError();
-}
-
-// The driver's tensor-map encoder (cuTensorMapEncodeTiled), or null.
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
-                                         &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  }();
-  return fn;
-}
-
-// The column-pass output of a batch as floats [batch][G/2 + 1][2 N], in boxes
-// of 4 floats (rows yy1, yy1 + 1 of a column) x kBandBox columns.
-static bool encode_band_map(CUtensorMap* m, const float2* colbuf, const FipGeom& geo, int batch,
-                            size_t col_stride) {
-  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-  if (!enc || ((uintptr_t)colbuf & 15) != 0 || batch < 1) return false;
-  const cuuint64_t dims[3] = {2 * (cuuint64_t)geo.n, (cuuint64_t)geo.hp, (cuuint64_t)batch};
-  const cuuint64_t strides[2] = {2 * (cuuint64_t)geo.n * 4,
-                                 (cuuint64_t)(batch > 1 ? col_stride : (size_t)geo.hp * geo.n) * 8};
-  const cuuint32_t box[3] = {4, (cuuint32_t)kBandBox, 1};
-  const cuuint32_t es[3] = {1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float2*>(colbuf), dims, strides,
-             box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
-         CUDA_SUCCESS;
-}
-
-template <int LM, int LE>
-static cudaError_t launch_rows(const FipGeom& geo, const float2* colbuf, unsigned* bbox,
-                               const float* taper, const float2* tw, float* pre,
-                               cudaStream_t s, int batch, size_t col_stride,
-                               size_t pre_stride, int split, int direct) {
-  size_t smem;
-  cudaError_t e;
-  const CUtensorMap no_map{};
-  if (split) {
-    smem = 2 * (size_t)fipfft::sub_stride(1 << LM) * sizeof(float2);
-    if ((e = fft_smem_attr((const void*)k_fft_rows_split<LM, LE>, smem)) != cudaSuccess)
-      return e;
-    k_fft_rows_split<LM, LE><<<dim3(geo.n / 2, 3, batch), split_threads<LM, LE>(), smem, s>>>(
-        colbuf, bbox, taper + geo.n / 2 + 1, pre, tw, col_stride, pre_stride);
-    return cudaGetLastError();
-  }
-  CUtensorMap band_map{};
-  if (direct == 2 && encode_band_map(&band_map, colbuf, geo, batch, col_stride)) {
-    // Persistent over row pairs (the CTAs that fit at once), the band copy
-    // one row pair ahead.
-    smem = band_smem_bytes<LM>();
-    e = fft_smem_attr((const void*)k_fft_rows<LM, LE, true, true>, smem);
-    if (e != cudaSuccess) return e;
-    static const int per_sm = [&] {
-      int v = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_fft_rows<LM, LE, true, true>,
-                                                        fft_threads<LM, LE>(), smem) !=
-          cudaSuccess)
-        v = 1;
-      return std::max(v, 1);
-    }();
-    const int ctas = std::max(1, std::min(geo.n / 2, per_sm * sm_count()));
-    k_fft_rows<LM, LE, true, true><<<dim3(ctas, batch), fft_threads<LM, LE>(), smem, s>>>(
-        colbuf, bbox, taper + geo.n / 2 + 1, pre, tw, col_stride, pre_stride, band_map);
-    return cudaGetLastError();
-  }
-  if (direct) {
-    smem = (size_t)fipfft::direct_smem_elems(geo.g) * sizeof(float2);
-    e = fft_smem_attr((const void*)k_fft_rows<LM, LE, true>, smem);
-    if (e != cudaSuccess) return e;
-    k_fft_rows<LM, LE, true><<<dim3(geo.n / 2, batch), fft_threads<LM, LE>(), smem, s>>>(
-        colbuf, bbox, taper + geo.n / 2 + 1, pre, tw, col_stride, pre_stride, no_map);
-    return cudaGetLastError();
-  }
-  smem = (size_t)fipfft::smem_elems(geo.g) * sizeof(float2);
-  e = fft_smem_attr((const void*)k_fft_rows<LM, LE, false>, smem);
-  if (e != cudaSuccess) return e;
-  // Persistent over row pairs: the CTAs that fit at once.
-  // (Queried once per instantiation: the shape and shared memory are fixed by it.)
-  static const int per_sm = [&] {
-    int v = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k_fft_rows<LM, LE, false>,
-                                                      fft_threads<LM, LE>(), smem) != cudaSuccess)
-      v = 1;
-    return std::max(v, 1);
-  }();
-  const int ctas = std::max(1, std::min(geo.n / 2, per_sm * sm_count()));
-  k_fft_rows<LM, LE, false><<<dim3(ctas, batch), fft_threads<LM, LE>(), smem, s>>>(
-      colbuf, bbox, taper + geo.n / 2 + 1, pre, tw, col_stride, pre_stride, no_map);
-  return cudaGetLastError();
-}
-
-// Calls F<LM, LE> for the plan's instantiation.
-#define FIP_FFT_SWITCH(PLAN, CALL)                                      \
-  do {                                                                  \
-    const int key_ = (PLAN).lm * 8 + (PLAN).le;                         \
-    switch (key_) {                                                     \
-      case 4 * 8 + 3: { constexpr int LM_ = 4, LE_ = 3; return CALL; }  \
-      case 5 * 8 + 3: { constexpr int LM_ = 5, LE_ = 3; return CALL; }  \
-      case 6 * 8 + 3: { constexpr int LM_ = 6, LE_ = 3; return CALL; }  \
-      case 7 * 8 + 3: { constexpr int LM_ = 7, LE_ = 3; return CALL; }  \
-      case 8 * 8 + 3: { constexpr int LM_ = 8, LE_ = 3; return CALL; }  \
-      case 9 * 8 + 3: { constexpr int LM_ = 9, LE_ = 3; return CALL; }  \
-      case 10 * 8 + 3: { constexpr int LM_ = 10, LE_ = 3; return CALL; } \
-      case 11 * 8 + 3: { constexpr int LM_ = 11, LE_ = 3; return CALL; } \
-      case 5 * 8 + 4: { constexpr int LM_ = 5, LE_ = 4; return CALL; }  \
-      case 6 * 8 + 4: { constexpr int LM_ = 6, LE_ = 4; return CALL; }  \
-      case 7 * 8 + 4: { constexpr int LM_ = 7, LE_ = 4; return CALL; }  \
-      case 8 * 8 + 4: { constexpr int LM_ = 8, LE_ = 4; return CALL; }  \
-      case 9 * 8 + 4: { constexpr int LM_ = 9, LE_ = 4; return CALL; }  \
-      case 10 * 8 + 4: { constexpr int LM_ = 10, LE_ = 4; return CALL; } \
-      case 11 * 8 + 4: { constexpr int LM_ = 11, LE_ = 4; return CALL; } \
-      case 12 * 8 + 4: { constexpr int LM_ = 12, LE_ = 4; return CALL; } \
-      default: return cudaErrorInvalidValue;                             \
-    }                                                                   \
-  } while (0)
-
-cudaError_t fip_launch_fft_cols(const FipGeom& geo, const float2* grid, const unsigned* bbox,
-                                float2* colbuf, const float2* twiddles, const fipfft::Plan& plan,
-                                cudaStream_t s, int batch, size_t grid_stride,
-                                size_t col_stride) {
-  if (plan.g != geo.g || batch < 1 || batch > 65535) return cudaErrorInvalidValue;
-  FIP_FFT_SWITCH(plan, (launch_cols<LM_, LE_>(geo, grid, bbox, colbuf, twiddles, s, batch,
-                                              grid_stride, col_stride, plan.split,
-                                              plan.direct)));
-}
-
-cudaError_t fip_launch_fft_rows(const FipGeom& geo, const float2* colbuf, unsigned* bbox,
-                                const float* taper, const float2* twiddles,
-                                const fipfft::Plan& plan, float* pre, cudaStream_t s, int batch,
-                                size_t col_stride, size_t pre_stride) {
-  if (plan.g != geo.g || batch < 1 || batch > 65535) return cudaErrorInvalidValue;
-  FIP_FFT_SWITCH(plan, (launch_rows<LM_, LE_>(geo, colbuf, bbox, taper, twiddles, pre, s, batch,
-                                              col_stride, pre_stride, plan.split,
-                                              plan.direct)));
-}
-
-cudaError_t fip_launch_correct_c2r(const FipGeom& geo, const float* fft_out, const float* taper,
-                                   float* pre, unsigned* pre_max, cudaStream_t s) {
-  dim3 bl((geo.n + kThreads - 1) / kThreads, geo.n);
-  k_correct_c2r<<<bl, kThreads, 0, s>>>(fft_out, taper, geo.n, geo.g, pre, pre_max);
-  return cudaGetLastError();
-}
-
-const void* fip_targets_kernel() { return reinterpret_cast<const void*>(&k_targets); }
+const void* fip_targets_kernel() { return reinterpret_cast<const void*>(&k_targets<false>); }
 
 cudaError_t fip_launch_targets(const FipGeom& geo, const float* V, const float2* theta_tab,
-                               float2* targets, cudaStream_t s) {
+                               float2* targets, cudaStream_t s, int batch, size_t stride) {
+  if (batch < 1 || batch > 65535) return cudaErrorInvalidValue;
   const int per = kThreads * kTargetsPerThread;
-  dim3 bl((geo.n + per - 1) / per, geo.n);
-  k_targets<<<bl, kThreads, 0, s>>>(V, geo.n, cell_degrees(geo.cell), theta_tab, targets);
+  dim3 bl((geo.n + per - 1) / per, geo.n, batch);
+  auto kern = batch > 1 ? k_targets<true> : k_targets<false>;
+  kern<<<bl, kThreads, 0, s>>>(V, geo.n, cell_degrees(geo.cell), theta_tab, targets, stride);
   return cudaGetLastError();
 }
 
@@ -2649,13 +1969,13 @@ size_t fip_trigger_fuse_counts(const FipGeom& geo) {
   return tiles * tiles;
 }
 
-cudaError_t fip_launch_reproject_gather(const FipGeom& geo, const float* pre,
-                                        const float2* targets, const float* V, int nb,
-                                        const unsigned* pre_max, float* dst, unsigned* img_max,
-                                        int exact_targets, cudaStream_t s, unsigned* err,
-                                        const FipFuse* fuse) {
+cudaError_t fip_launch_reproject_gather(const FipGeom& geo, const FipGatherBatch& in,
+                                        const float* pre, const float2* targets,
+                                        const unsigned* pre_max, int exact_targets,
+                                        cudaStream_t s, unsigned* err, const FipFuse* fuse) {
   const int tiles = (geo.n + kDT - 1) / kDT;
   const float delta = exact_targets ? 0.25f : chain_delta(geo.cell);
+  if (in.count < 1 || in.count > FIP_MAX_BATCH) return cudaErrorInvalidValue;
   if (!fip_gather_supported(geo, exact_targets)) return cudaErrorInvalidValue;
   FipTriggerFuse tf{};
   if (fuse) {
@@ -2666,12 +1986,13 @@ cudaError_t fip_launch_reproject_gather(const FipGeom& geo, const float* pre,
     tf.t = geo.t;
     tf.u = geo.u;
   }
-  if (exact_targets)
-    k_reproject_gather<true><<<tiles * tiles, kThreads, 0, s>>>(
-        pre, nullptr, V, geo.n, nb, geo.cell, delta, pre_max, dst, img_max, err, tf);
-  else
-    k_reproject_gather<false><<<tiles * tiles, kThreads, 0, s>>>(
-        pre, targets, V, geo.n, nb, geo.cell, delta, pre_max, dst, img_max, err, tf);
+  const dim3 blocks(tiles * tiles, in.count);
+  const float2* tg = exact_targets ? nullptr : targets;
+  auto kern = exact_targets
+                  ? (in.count > 1 ? k_reproject_gather<true, true> : k_reproject_gather<true, false>)
+                  : (in.count > 1 ? k_reproject_gather<false, true>
+                                  : k_reproject_gather<false, false>);
+  kern<<<blocks, kThreads, 0, s>>>(in, pre, tg, geo.n, geo.cell, delta, pre_max, err, tf);
   return cudaGetLastError();
 }
 
@@ -2768,11 +2089,26 @@ cudaError_t fip_launch_trigger3(const FipGeom& geo, const float* I1, const float
   const int vec = (geo.t % 4 == 0) && (geo.n % 4 == 0) &&
                   ((((uintptr_t)I1) | ((uintptr_t)I2) | ((uintptr_t)I3)) & 15) == 0;
   if (precise)
-    k_trigger<true><<<blocks, kThreads, 0, s>>>(I1, I2, I3, m1, m2, m3, geo.n, geo.t, geo.u, vec,
-                                                result, 0, 0);
+    k_trigger<true, false><<<blocks, kThreads, 0, s>>>(I1, I2, I3, m1, m2, m3, geo.n, geo.t, geo.u, vec,
+                                                result, 0, 0, 0, 0);
   else
-    k_trigger<false><<<blocks, kThreads, 0, s>>>(I1, I2, I3, m1, m2, m3, geo.n, geo.t, geo.u,
-                                                 vec, result, 0, 0);
+    k_trigger<false, false><<<blocks, kThreads, 0, s>>>(I1, I2, I3, m1, m2, m3, geo.n, geo.t, geo.u,
+                                                 vec, result, 0, 0, 0, 0);
+  return cudaGetLastError();
+}
+
+cudaError_t fip_launch_trigger_ring(const FipGeom& geo, const float* images, const float* maxima,
+                                    int ring, int first, int count, float* results, int precise,
+                                    cudaStream_t s) {
+  const int tiles = geo.u * geo.u;
+  if (tiles == 0 || count <= 0) return cudaSuccess;
+  if (count > 65535 || ring < 3) return cudaErrorInvalidValue;
+  const size_t n2 = (size_t)geo.n * geo.n;
+  const dim3 blocks((tiles + kThreads / 32 - 1) / (kThreads / 32), count);
+  const int vec = (geo.t % 4 == 0) && (geo.n % 4 == 0) && ((uintptr_t)images & 15) == 0;
+  auto kern = precise ? k_trigger<true, true> : k_trigger<false, true>;
+  kern<<<blocks, kThreads, 0, s>>>(images, images, images, maxima, maxima, maxima, geo.n, geo.t,
+                                   geo.u, vec, results, n2, (size_t)tiles, ring, first);
   return cudaGetLastError();
 }
 
@@ -2791,13 +2127,13 @@ cudaError_t fip_launch_trigger_batch(const FipGeom& geo, const float* images, co
   const dim3 blocks((tiles + kThreads / 32 - 1) / (kThreads / 32), count);
   const int vec = (geo.t % 4 == 0) && (geo.n % 4 == 0) && ((uintptr_t)images & 15) == 0;
   if (precise)
-    k_trigger<true><<<blocks, kThreads, 0, s>>>(images, images + n2, images + 2 * n2, maxima,
+    k_trigger<true, false><<<blocks, kThreads, 0, s>>>(images, images + n2, images + 2 * n2, maxima,
                                                 maxima + 1, maxima + 2, geo.n, geo.t, geo.u, vec,
-                                                results, n2, (size_t)tiles);
+                                                results, n2, (size_t)tiles, 0, 0);
   else
-    k_trigger<false><<<blocks, kThreads, 0, s>>>(images, images + n2, images + 2 * n2, maxima,
+    k_trigger<false, false><<<blocks, kThreads, 0, s>>>(images, images + n2, images + 2 * n2, maxima,
                                                  maxima + 1, maxima + 2, geo.n, geo.t, geo.u,
-                                                 vec, results, n2, (size_t)tiles);
+                                                 vec, results, n2, (size_t)tiles, 0, 0);
   return cudaGetLastError();
 }
 

@@ -371,21 +371,29 @@ struct F32Vis {
     re = vr[k];
     im = vi[k];
   }
+  __device__ __forceinline__ F32Vis at(size_t off) const { return F32Vis{vr + off, vi + off}; }
 };
 struct RawVis {
   FipRawVis r;
   __device__ __forceinline__ void operator()(size_t k, float& re, float& im) const {
     fip_collapse_sample(r, k, re, im);
   }
+  __device__ __forceinline__ RawVis at(size_t) const { return *this; }  // one snapshot per launch
 };
 
 // One block of FIP_QBLOCK samples per CTA (kThreads threads, four samples
 // each): the block's max-abs, its power-of-two scale 2^(e - 14) for a max-abs
 // in [2^e, 2^(e+1)) (so the max lands in [2^14, 2^15), inside FP16's range,
 // and the division by the scale is exact), then the values divided by it.
+// Batched launches: snapshot blockIdx.y.
 template <int VT, class L>
-__global__ void __launch_bounds__(kThreads) k_quantize(const L load, size_t nb, void* qr,
-                                                       void* qi, float* scales) {
+__global__ void __launch_bounds__(kThreads) k_quantize(const L load0, size_t nb, void* qr,
+                                                       void* qi, float* scales,
+                                                       size_t in_stride, size_t out_stride) {
+  const L load = load0.at(blockIdx.y * in_stride);
+  qr = static_cast<uint16_t*>(qr) + blockIdx.y * out_stride;
+  qi = static_cast<uint16_t*>(qi) + blockIdx.y * out_stride;
+  scales += blockIdx.y * fip_qblocks(out_stride);
   static_assert(FIP_QBLOCK == 4 * kThreads, "four samples per thread");
   __shared__ float s_max[kThreads / 32];
   const size_t base = (size_t)blockIdx.x * FIP_QBLOCK;
@@ -468,21 +476,26 @@ cudaError_t fip_launch_collapse(const float* v0r, const float* v0i, const float*
 
 template <class L>
 static cudaError_t launch_quantize(const L& load, size_t nb, int vis_type, void* out_re,
-                                  void* out_im, float* scales, cudaStream_t s) {
+                                  void* out_im, float* scales, cudaStream_t s, int batch = 1,
+                                  size_t in_stride = 0, size_t out_stride = 0) {
   const size_t blocks = fip_qblocks(nb);
   if (blocks == 0) return cudaSuccess;
   if (blocks > 0x7fffffffu) return cudaErrorInvalidValue;
   if (vis_type == FIP_VIS_F16)
-    k_quantize<FIP_VIS_F16><<<(unsigned)blocks, kThreads, 0, s>>>(load, nb, out_re, out_im, scales);
+    k_quantize<FIP_VIS_F16><<<dim3((unsigned)blocks, batch), kThreads, 0, s>>>(
+        load, nb, out_re, out_im, scales, in_stride, out_stride);
   else
-    k_quantize<FIP_VIS_BF16><<<(unsigned)blocks, kThreads, 0, s>>>(load, nb, out_re, out_im,
-                                                                   scales);
+    k_quantize<FIP_VIS_BF16><<<dim3((unsigned)blocks, batch), kThreads, 0, s>>>(
+        load, nb, out_re, out_im, scales, in_stride, out_stride);
   return cudaGetLastError();
 }
 
 cudaError_t fip_launch_quantize(const float* vr, const float* vi, size_t nb, int vis_type,
-                                void* out_re, void* out_im, float* scales, cudaStream_t s) {
-  return launch_quantize(F32Vis{vr, vi}, nb, vis_type, out_re, out_im, scales, s);
+                                void* out_re, void* out_im, float* scales, cudaStream_t s,
+                                int batch, size_t in_stride, size_t out_stride) {
+  if (batch < 1 || batch > 65535) return cudaErrorInvalidValue;
+  return launch_quantize(F32Vis{vr, vi}, nb, vis_type, out_re, out_im, scales, s, batch,
+                         in_stride, out_stride);
 }
 
 cudaError_t fip_launch_quantize_raw(const FipRawVis& raw, size_t nb, int vis_type, void* out_re,
