@@ -2,10 +2,11 @@
 
     python -m fastimagingpipe_b200.build
 
-Compiles every CUDA translation unit for sm_100a only.  fip_plain.cu and
-fip_transform.cu get --use_fast_math (the reference's own build flags: the
-plain form reproduces its FP32 arithmetic); the other units are IEEE.  Objects go to
-fastimagingpipe_b200/_build/, the library and the CLI next to this file.
+Compiles every CUDA translation unit for sm_100a only.  fip_plain.cu,
+fip_transform.cu and fip_pull.cu get --use_fast_math (the reference's own build
+flags: the plain form reproduces its FP32 arithmetic); the other units are
+IEEE.  Objects go to fastimagingpipe_b200/_build/, the library and the CLI next
+to this file.
 """
 from __future__ import annotations
 
@@ -28,6 +29,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 UNITS = {
     "fip_plain.cu": ["--use_fast_math"],
     "fip_transform.cu": ["--use_fast_math"],
+    "fip_pull.cu": ["--use_fast_math"],
     "fip_precise.cu": [],
     "fip_host.cu": [],
     "fip_noalloc.cu": [],

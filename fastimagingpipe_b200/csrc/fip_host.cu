@@ -259,6 +259,7 @@ struct Lane {
   float2* colbuf = nullptr;          // column-pass output [G/2+1][N]
   float* pre = nullptr;              // corrected pre-reprojection image [N*N]
   float2* targets = nullptr;         // reference pixel mapping [N*N]
+  unsigned* plans = nullptr;         // the precision form's pull plans, or null: it splats
   void* q_re = nullptr;              // reduced-precision visibility storage
   void* q_im = nullptr;
   float* q_scale = nullptr;
@@ -572,6 +573,8 @@ int fip_imager_create(fip_imager** out, const fip_imager_config* cfg) {
   FIP_LANES(bins.nmulti, 1);
   FIP_LANES(pre, n2);
   if (cfg->form == FIP_FORM_PLAIN && cfg->reproject == 0) FIP_LANES(targets, n2);
+  if (cfg->form == FIP_FORM_PRECISE && cfg->reproject == 0 && fip_pull_supported(geo))
+    FIP_LANES(plans, fip_pull_plan_words(geo));
   if (im->custom_fft) FIP_LANES(colbuf, im->col_stride);
   if (cfg->form == FIP_FORM_PRECISE && cfg->vis_storage != FIP_STORE_F32) {
     uint16_t *qr = nullptr, *qi = nullptr;
@@ -684,19 +687,29 @@ static int image_snapshot_impl(fip_imager* im, Lane& L, const float* vr, const f
   // force_scatter: the snapshot's geometry lies outside the gather's domain
   // (checked on the host where V is a host array): the reference's scheme.
   const bool gather = im->cfg.reproject == 0 && !force_scatter;
-  const bool chain_targets = gather && !precise;
-  // The pixel mapping depends on V only: it may run beside gridding + FFT on
-  // the side stream (serialised on s when profiling, so every stage's time
-  // is its own).
-  const bool fork = chain_targets && fork_targets && !im->timer.on;
-  if (chain_targets && !targets_ready) {
+  // What the reprojection needs of the plane, V, alone -- the pixel mapping or
+  // the pull's plan -- may run beside gridding + FFT on the side stream
+  // (serialised on s when profiling, so every stage's time is its own).
+  const bool pull = gather && L.plans;
+  const bool plane_work = gather && (!precise || pull);
+  const bool fork = plane_work && fork_targets && !targets_ready && !im->timer.on;
+  FipGatherBatch gb;
+  gb.count = 1;
+  gb.V[0] = V;
+  gb.nb[0] = (int)nb;
+  gb.dst[0] = image;
+  gb.img_max[0] = reinterpret_cast<unsigned*>(image_max);
+  if (plane_work && !targets_ready) {
     cudaStream_t ts = fork ? im->side : s;
     if (fork) {
       FIP_CUDA(cudaEventRecord(im->ev_fork, s));
       FIP_CUDA(cudaStreamWaitEvent(im->side, im->ev_fork, 0));
     }
     k = stage_begin(im, ST_TARGETS, ts);
-    FIP_CUDA(fip_launch_targets(geo, V, im->theta_tab, L.targets, ts));
+    if (pull)
+      FIP_CUDA(fip_launch_pull_plan(geo, gb, L.plans, ts));
+    else
+      FIP_CUDA(fip_launch_targets(geo, V, im->theta_tab, L.targets, ts));
     stage_end(im, k, ts);
     im->launches += 1;
     if (fork) FIP_CUDA(cudaEventRecord(im->ev_join, im->side));
@@ -759,16 +772,13 @@ static int image_snapshot_impl(fip_imager* im, Lane& L, const float* vr, const f
     if (fork) FIP_CUDA(cudaStreamWaitEvent(s, im->ev_join, 0));
     if (targets_ready && targets_ev) FIP_CUDA(cudaStreamWaitEvent(s, targets_ev, 0));
     k = stage_begin(im, ST_REPROJECT, s);
-    FipGatherBatch in;
-    in.count = 1;
-    in.V[0] = V;
-    in.nb[0] = (int)nb;
-    in.dst[0] = image;
-    in.img_max[0] = reinterpret_cast<unsigned*>(image_max);
-    FIP_CUDA(fip_launch_reproject_gather(geo, in, L.pre, L.targets, L.bins.bbox + 3,
-                                         precise ? 1 : 0, s, im->gather_err, fuse));
+    if (pull)
+      FIP_CUDA(fip_launch_pull(geo, gb, L.pre, L.plans, L.bins.bbox + 3, s, im->gather_err));
+    else
+      FIP_CUDA(fip_launch_reproject_gather(geo, gb, L.pre, L.targets, L.bins.bbox + 3,
+                                           precise ? 1 : 0, s, im->gather_err, fuse));
     stage_end(im, k, s);
-    im->launches += 1;
+    im->launches += pull ? 2 : 1;
   }
   return FIP_OK;
 }
@@ -814,19 +824,35 @@ static FipFuse fuse_of(const fip_imager* im) {
   return f;
 }
 
-// Whether a three-snapshot call maps its pixels ahead on the side stream:
-// concurrent lanes, the gather reprojection of the plain form (the precision
-// form evaluates the exact map inside the gather).
+// Whether a three-snapshot call does its reprojections' plane work ahead on the
+// side stream: concurrent lanes, and the plain form's pixel mappings or the
+// precision form's pull plans.
 static bool targets_ahead(const fip_imager* im) {
   return im->lanes > 1 && !im->timer.on && im->cfg.reproject == 0 &&
-         im->cfg.form == FIP_FORM_PLAIN;
+         (im->cfg.form == FIP_FORM_PLAIN || im->lane[0].plans);
 }
 
-// The pixel mappings of a call's three snapshots (bases V + 9 k), on the
+// The pull plans of `count` snapshots (bases V + 9 k) into lanes 0 .. count - 1.
+static int launch_plans(fip_imager* im, const float* V, int count, cudaStream_t s) {
+  FipGatherBatch gb{};
+  gb.count = count;
+  for (int k = 0; k < count; ++k) gb.V[k] = V + (size_t)k * 9;
+  FIP_CUDA(fip_launch_pull_plan(im->geo, gb, im->lane[0].plans, s));
+  im->launches += 1;
+  return FIP_OK;
+}
+
+// The plane work of a call's three snapshots (bases V + 9 k), on the
 // low-priority side stream after `after`; lane k's gather waits on its
 // ev_targets.
 static int launch_targets_ahead(fip_imager* im, const float* V, cudaEvent_t after) {
   FIP_CUDA(cudaStreamWaitEvent(im->side, after, 0));
+  if (im->cfg.form == FIP_FORM_PRECISE) {
+    FIP_TRY(launch_plans(im, V, 3, im->side));
+    for (int k = 0; k < 3; ++k)
+      FIP_CUDA(cudaEventRecord(im->lane[k % im->lanes].ev_targets, im->side));
+    return FIP_OK;
+  }
   for (int k = 0; k < 3; ++k) {
     Lane& L = im->lane[k % im->lanes];
     FIP_CUDA(fip_launch_targets(im->geo, V + (size_t)k * 9, im->theta_tab, L.targets, im->side));
@@ -868,12 +894,16 @@ static int image_merged(fip_imager* im, int count, const float* vr, const float*
   const size_t n2 = (size_t)geo.n * geo.n;
   Lane& L = im->lane[0];
   FIP_CUDA(cudaMemsetAsync(im->zero_block, 0, im->zero_words * sizeof(unsigned), s));
-  // The pixel mappings need only V: beside everything up to the reprojection
-  // (on s itself, at 512^2, 83 against 76 us a call).
-  if (!precise) {
+  // The pixel mappings (or pull plans) need only V: beside everything up to the
+  // reprojection (on s itself, at 512^2, 83 against 76 us a plain call).
+  const bool plane_work = !precise || L.plans;
+  if (plane_work) {
     FIP_CUDA(cudaEventRecord(im->ev_fork, s));
     FIP_CUDA(cudaStreamWaitEvent(im->side, im->ev_fork, 0));
-    FIP_CUDA(fip_launch_targets(geo, V, im->theta_tab, L.targets, im->side, count, n2));
+    if (precise)
+      FIP_TRY(launch_plans(im, V, count, im->side));
+    else
+      FIP_CUDA(fip_launch_targets(geo, V, im->theta_tab, L.targets, im->side, count, n2));
     FIP_CUDA(cudaEventRecord(im->ev_join, im->side));
   }
   FipBinBatch bin;
@@ -929,9 +959,14 @@ static int image_merged(fip_imager* im, int count, const float* vr, const float*
                                im->grid_stride, im->col_stride));
   FIP_CUDA(fip_launch_fft_rows(geo, L.colbuf, L.bins.bbox, im->taper, im->twiddles, im->fft,
                                L.pre, s, count, im->col_stride, n2));
-  if (!precise) FIP_CUDA(cudaStreamWaitEvent(s, im->ev_join, 0));
-  FIP_CUDA(fip_launch_reproject_gather(geo, gb, L.pre, L.targets, L.bins.bbox + 3,
-                                       precise ? 1 : 0, s, im->gather_err, fuse));
+  if (plane_work) FIP_CUDA(cudaStreamWaitEvent(s, im->ev_join, 0));
+  if (L.plans) {
+    FIP_CUDA(fip_launch_pull(geo, gb, L.pre, L.plans, L.bins.bbox + 3, s, im->gather_err));
+    im->launches += 1;
+  } else {
+    FIP_CUDA(fip_launch_reproject_gather(geo, gb, L.pre, L.targets, L.bins.bbox + 3,
+                                         precise ? 1 : 0, s, im->gather_err, fuse));
+  }
   im->launches += precise ? 7 : 8;  // binning 3, grid, transforms 2, gather (and mapping)
   im->last_lane = count - 1;
   return FIP_OK;
@@ -1587,6 +1622,7 @@ struct BatchSeq {
   float2* colbuf = nullptr;           // [smax][(G/2+1) N]
   float* pre = nullptr;               // [smax][N N]
   float2* targets = nullptr;          // [smax][N N] (plain form)
+  unsigned* pull_plans = nullptr;     // [smax][plan] (precision form's pull, or null)
   void* q_re = nullptr;               // [smax][max_baselines] (reduced storage)
   void* q_im = nullptr;
   float* q_scale = nullptr;           // [smax][fip_qblocks(max_baselines)]
@@ -1621,7 +1657,7 @@ struct BatchSeq {
     for (auto& p : plans) cufftDestroy(p.second);
     plans.clear();
     void* ptrs[] = {twiddles, taper, count, offset, cursor, entries, work, nwork, bbox, multi,
-                    nmulti, grid, colbuf, pre, targets, q_re, q_im, q_scale, images, maxima};
+                    nmulti, grid, colbuf, pre, targets, pull_plans, q_re, q_im, q_scale, images, maxima};
     for (void* p : ptrs)
       if (p) cudaFree(p);
   }
@@ -1788,6 +1824,29 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
     for (int i = 0; i < fip_batch::kMapBranches; ++i)
       FIP_CUDA(cudaEventRecord(b->map_join[i], b->map_branch[i]));
   }
+  // The reprojection of sequence c's snapshots: into ring slots 2 ..
+  // count + 1 (or the caller's slots).
+  auto gather_batch = [&](int c) {
+    const BatchSeq& q = b->seq[c];
+    FipGatherBatch gb;
+    gb.count = l.per[c];
+    for (int k = 0; k < count; ++k) {
+      if (l.sq[k] != c) continue;
+      const int j = l.loc[k];
+      gb.V[j] = V[k];
+      gb.nb[j] = (int)nb[k];
+      gb.dst[j] = slots ? slots[k].image : q.images + (j + 2) * q.n2;
+      gb.img_max[j] = reinterpret_cast<unsigned*>(slots ? slots[k].image_max : q.maxima + j + 2);
+    }
+    return gb;
+  };
+  // The precision form's pull plans, beside the conversion and binning.
+  for (int c = 0; c < nseq; ++c) {
+    const BatchSeq& q = b->seq[c];
+    if (l.per[c] == 0 || !q.pull_plans) continue;
+    FIP_CUDA(fip_launch_pull_plan(q.geo, gather_batch(c), q.pull_plans, b->branch[c % kBranches]));
+    launches += 1;
+  }
   FipGridBatch in{};
   in.count = count;
   FipBinBatch joint;
@@ -1887,15 +1946,11 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
     if (l.per[c] == 0) continue;
     cudaStream_t bs = b->branch[c % kBranches];
     FIP_CUDA(cudaStreamWaitEvent(bs, b->fork, 0));
-    FipGatherBatch gb;
-    gb.count = l.per[c];
-    for (int k = 0; k < count; ++k) {
-      if (l.sq[k] != c) continue;
-      const int j = l.loc[k];
-      gb.V[j] = V[k];
-      gb.nb[j] = (int)nb[k];
-      gb.dst[j] = slots ? slots[k].image : q.images + (j + 2) * q.n2;
-      gb.img_max[j] = reinterpret_cast<unsigned*>(slots ? slots[k].image_max : q.maxima + j + 2);
+    const FipGatherBatch gb = gather_batch(c);
+    if (q.pull_plans) {
+      FIP_CUDA(fip_launch_pull(q.geo, gb, q.pre, q.pull_plans, q.bbox + 3, bs, b->gather_err));
+      launches += 2;
+      continue;
     }
     FIP_CUDA(fip_launch_reproject_gather(q.geo, gb, q.pre, precise ? nullptr : q.targets,
                                          q.bbox + 3, precise ? 1 : 0, bs, b->gather_err));
@@ -1996,6 +2051,8 @@ int seq_alloc(BatchSeq& q, size_t smax, size_t& tot) {
   if (q.custom_fft) FIP_SALLOC(dalloc(&q.colbuf, S * q.col_elems, tot));
   FIP_SALLOC(dalloc(&q.pre, S * q.n2, tot));
   if (cfg.form == FIP_FORM_PLAIN) FIP_SALLOC(dalloc(&q.targets, S * q.n2, tot));
+  if (cfg.form == FIP_FORM_PRECISE && fip_pull_supported(geo))
+    FIP_SALLOC(dalloc(&q.pull_plans, S * fip_pull_plan_words(geo), tot));
   if (cfg.form == FIP_FORM_PRECISE && cfg.vis_storage != FIP_STORE_F32) {
     FIP_SALLOC(dalloc((uint16_t**)&q.q_re, S * nb, tot));
     FIP_SALLOC(dalloc((uint16_t**)&q.q_im, S * nb, tot));

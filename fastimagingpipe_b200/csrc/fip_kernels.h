@@ -134,6 +134,26 @@ cudaError_t fip_launch_reproject_gather(const FipGeom& geo, const FipGatherBatch
                                         const unsigned* pre_max, int exact_targets,
                                         cudaStream_t s, unsigned* err,
                                         const FipFuse* fuse = nullptr);
+// The precision form's reprojection by destination pixel (fip_pull.cu), for
+// images of at least kPullMin pixels a side with cells of at most kPullCell: the
+// plan depends on the bases in.V only ([count][fip_pull_plan_words] words) and
+// may run ahead; the pull writes the tiles the plan covers, then splats the
+// rest (fip_launch_reproject_rest).  Smaller images gain nothing over the splat (a
+// 512^2 call 78 us either way: latency); wider cells leave the plan's range.
+constexpr int kPullMin = 768;
+constexpr float kPullCell = 4e-5f;
+bool fip_pull_supported(const FipGeom& geo);
+size_t fip_pull_plan_words(const FipGeom& geo);
+cudaError_t fip_launch_pull_plan(const FipGeom& geo, const FipGatherBatch& in, unsigned* plans,
+                                 cudaStream_t s);
+cudaError_t fip_launch_pull(const FipGeom& geo, const FipGatherBatch& in, const float* pre,
+                            const unsigned* plans, const unsigned* pre_max, cudaStream_t s,
+                            unsigned* err);
+// The splat (fip_launch_reproject_gather, exact targets) over the tiles whose
+// plan has no rows.
+cudaError_t fip_launch_reproject_rest(const FipGeom& geo, const FipGatherBatch& in,
+                                      const float* pre, const unsigned* plans,
+                                      const unsigned* pre_max, cudaStream_t s, unsigned* err);
 // Whether the plane-to-sky map of basis V (host, row-major 3 x 3) stays in
 // the tile gather's domain over an N x N image: well inside the horizon and
 // without folds.  Outside it only the source scatter reprojects correctly.

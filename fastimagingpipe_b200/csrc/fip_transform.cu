@@ -2,9 +2,7 @@
 // crop-and-correction epilogue, and the crop of cuFFT's output for the
 // remaining grid sides.  Compiled with --use_fast_math like the other stages
 // of the plain form (fip_plain.cu).
-#include <cuda.h>
 #include <cuda_runtime.h>
-#include <cudaTypedefs.h>
 #include <stdint.h>
 
 #include <algorithm>
@@ -12,6 +10,7 @@
 #include "fip_common.cuh"
 #include "fip_fft.cuh"
 #include "fip_kernels.h"
+#include "fip_tma.cuh"
 
 namespace {
 
@@ -128,44 +127,6 @@ __global__ void __launch_bounds__(fft_threads<LM, LE>(), (fft_min_blocks<LM, LE,
   }
 }
 
-// Bulk tensor copies (TMA) with an mbarrier, for the row pass's band copy.
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-// Bounded wait for phase `parity` of *bar: false if it did not complete
-// within kMbarSpin polls.
-constexpr unsigned kMbarSpin = 1u << 20;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  const unsigned a = smem_u32(bar);
-  for (unsigned it = 0; it < kMbarSpin; ++it) {
-    unsigned done = 0;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y,
-                                            int z, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-}
 // The row pass's band copy: columns 0 .. K2 (at most kBandCap; wider bands
 // read global memory) of a row pair, kBandBox columns per bulk copy, 16
 // bytes (rows yy1, yy1 + 1 of one column) each.
@@ -600,22 +561,6 @@ static cudaError_t launch_cols(const FipGeom& geo, const float2* grid, const uns
   k_fft_cols<LM, LE, false><<<dim3(ctas, batch), fft_threads<LM, LE>(), smem, s>>>(
       grid, bbox, colbuf, tw, grid_stride, col_stride);
   return cudaGetLastError();
-}
-
-// The driver's tensor-map encoder (cuTensorMapEncodeTiled), or null.
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
-                                         &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  }();
-  return fn;
 }
 
 // The column-pass output of a batch as floats [batch][G/2 + 1][2 N], in boxes
