@@ -29,9 +29,12 @@ namespace fipfft {
 
 // Transform shape chosen on the host; the kernels are instantiated per
 // (lm, le), so the passes, radices and index arithmetic are compile-time.
+// any: M is not a power of two: run-time passes (fip_fft_any.cuh).
+constexpr int kMaxPasses = 12;
 struct Plan {
   int g;   // transform length G = 3 M
   int m;   // sub-transform length M = 2^lm
+  int any, passes, radix[kMaxPasses];
   int lm;  // log2 M
   int le;  // log2 of the complex values per thread (3 or 4)
   int e;   // values per thread

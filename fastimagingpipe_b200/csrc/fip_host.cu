@@ -1340,7 +1340,7 @@ int fip_imager_autotune(fip_imager* im, const float* vr, const float* vi, const 
     }
     return FIP_OK;
   };
-  if (im->custom_fft) {
+  if (im->custom_fft && !im->fft.any) {
     float best = 1e30f;
     fipfft::Plan chosen = im->fft;
     // Values per thread 8 or 16 x {joint, split, joint with a direct first
@@ -1395,7 +1395,7 @@ int fip_imager_set_tuning(fip_imager* im, int fft_values_per_thread, int fft_spl
   if (!im) return fail(FIP_ERR_ARG, "null imager");
   if (grid_ctas_per_sm < 0 || grid_ctas_per_sm > 8)
     return fail(FIP_ERR_ARG, "grid_ctas_per_sm must be in [0, 8]");
-  if (im->custom_fft) {
+  if (im->custom_fft && !im->fft.any) {
     fipfft::Plan p{};
     if (!fip_fft_plan(im->geo.g, p, fft_values_per_thread))
       return fail(FIP_ERR_ARG, "no transform with these values per thread for this size");
@@ -1603,7 +1603,7 @@ struct BatchSeq {
   FipGeom geo{};
   bool custom_fft = true;  // band-pruned transform; else batched cuFFT C2R plans
   fipfft::Plan fft{};
-  // cuFFT C2R plans by number of snapshots per call (grid sides not 3 * 2^k),
+  // cuFFT C2R plans by number of snapshots per call (sides the transforms lack),
   // created before the call's capture.
   std::vector<std::pair<int, cufftHandle>> plans;
   float2* twiddles = nullptr;
@@ -1892,7 +1892,7 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
   FIP_CUDA(fip_launch_grid_batch(in, vt, grid_compensated(precise, vt), s, b->grid_ctas_per_sm));
   launches += 1;
   FIP_CUDA(phase(2));
-  // Grid sides not 3 * 2^k: one batched cuFFT C2R (in place, phase 2) and the
+  // Sides the transforms lack: one batched cuFFT C2R (in place, phase 2) and the
   // crop + correction per snapshot (phase 3).
   for (int c = 0; c < nseq; ++c) {
     const BatchSeq& q = b->seq[c];
@@ -2018,7 +2018,7 @@ int seq_alloc(BatchSeq& q, size_t smax, size_t& tot) {
   geo.tiles_r = (geo.g + FIP_GTILE - 1) / FIP_GTILE;
   geo.tiles_c = (geo.hp + FIP_GTILE - 1) / FIP_GTILE;
   geo.cell = cfg.cell_size;
-  // The band-pruned transform (grid side 3 * 2^k, power-of-two images) works
+  // The band-pruned transforms work
   // on the band layout; other sides on the full grid with cuFFT.
   q.custom_fft = fip_fft_plan(geo.g, q.fft);
   geo.layout = q.custom_fft ? 1 : 0;
@@ -2447,7 +2447,7 @@ static int batch_autotune(fip_batch* b, const int* seq_of, const float* const* v
   };
   for (int c = 0; c < nseq; ++c) {
     BatchSeq& q = b->seq[c];
-    if (l.per[c] == 0 || !q.custom_fft) continue;
+    if (l.per[c] == 0 || !q.custom_fft || q.fft.any) continue;
     float best = 1e30f;
     fipfft::Plan chosen = q.fft;
     // Values per thread 8 or 16 x {joint, split, joint with a direct first

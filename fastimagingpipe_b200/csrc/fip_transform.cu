@@ -9,12 +9,25 @@
 
 #include "fip_common.cuh"
 #include "fip_fft.cuh"
+#include "fip_fft_any.cuh"
 #include "fip_kernels.h"
 #include "fip_tma.cuh"
 
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kAnyThreads = 256;
+// Run-time lengths: shared memory a CTA may take (sides up to 4,700), and the
+// largest prime factor of M they take.  A prime's pass costs in proportion to
+// it, cuFFT's convolution transform of the whole grid does not; both passes
+// against cuFFT's kernels and the crop, us: p = 199 at 796^2 37 and 44, at 2388^2
+// 208 and 370; p = 251 at 1004^2 53 and 66, p = 211 at 844^2 48 and 45; p =
+// 359 at 1436^2 152 and 120, p = 509 at 2036^2 328 and 225; p = 151 at
+// 3624^2 (whose grid cuFFT splits over several kernels) 551 (before four
+// outputs an item) and 1,069, p = 997 at 3988^2 about 2,250 and 1,512.
+constexpr int kAnySmem = 226 * 1024;
+constexpr int kAnyPrime = 509;
+static int any_prime_limit(int m) { return m >= 1500 ? kAnyPrime : (m >= 500 ? 251 : 199); }
 
 inline int sm_count() {
   int dev = 0, sms = 148;
@@ -457,8 +470,87 @@ __global__ void __launch_bounds__(split_threads<LM, LE>(), (LE == 4 ? 6 : 4))
   block_max_to(vmax, &bbox[3]);
 }
 
-// Crop + correction of the cuFFT C2R output (images whose grid side is not
-// 3 * 2^k): row (y mod G), column (x mod G), row stride G + 2 floats.
+// The two passes for run-time lengths (fip_fft_any.cuh): a CTA per column or row
+// pair in turn, several CTAs per SM hiding one another's barriers; inputs,
+// outputs and epilogue as the power-of-two passes'.  Bound: shared-memory
+// round trips and barriers.  Both passes against cuFFT's transform of the whole
+// grid and the crop, us: 1000^2 15 and 39, 1500^2 24 and 55, 3000^2 80 and 230,
+// 1484^2 (factor 53) 60 and 120; the band layout they allow also spares the
+// gridder the rest of the grid (3000^2 66 -> 45 us).
+__global__ void __launch_bounds__(kAnyThreads) k_fft_any_cols(const float2* __restrict__ H,
+                                                              const unsigned* __restrict__ bbox,
+                                                              float2* __restrict__ P,
+                                                              const float2* __restrict__ tw,
+                                                              const __grid_constant__ fipfft::Plan p,
+                                                              size_t grid_stride,
+                                                              size_t col_stride) {
+  extern __shared__ float2 s_fft[];
+  const int g = p.g, n = 2 * p.m, half = g / 2;
+  H += blockIdx.y * grid_stride;
+  P += blockIdx.y * col_stride;
+  bbox += 4 * blockIdx.y;
+  const int k2 = (int)bbox[1], k1 = min((int)bbox[0], half);
+  // Row -G/2 is row +G/2 (counted once).
+  const int lo = (k1 == half) ? 1 - k1 : -k1, hi = k1;
+  fipfft::any_load_roots(s_fft, p, tw);
+  for (int c = blockIdx.x; c <= k2; c += gridDim.x) {
+    const float2* col = H + (size_t)c * g;
+    fipfft::any_stage(s_fft, p, lo, hi, tw, [&](int r) { return col[r < 0 ? r + g : r]; });
+    __syncthreads();
+    const float2* y = fipfft::any_run(s_fft, p, tw);
+    float2* out = P + (size_t)c * n;
+    for (int o = threadIdx.x; o < n; o += blockDim.x) out[o] = fipfft::any_fetch(y, p.m, o);
+    __syncthreads();  // the next staging may write the buffer just read
+  }
+}
+
+__global__ void __launch_bounds__(kAnyThreads) k_fft_any_rows(const float2* __restrict__ P,
+                                                              unsigned* bbox,
+                                                              const float* __restrict__ rck,
+                                                              float* __restrict__ pre,
+                                                              const float2* __restrict__ tw,
+                                                              const __grid_constant__ fipfft::Plan p,
+                                                              size_t col_stride,
+                                                              size_t pre_stride) {
+  extern __shared__ float2 s_fft[];
+  const int n = 2 * p.m, half = p.g / 2, h = p.m;
+  P += blockIdx.y * col_stride;
+  pre += blockIdx.y * pre_stride;
+  bbox += 4 * blockIdx.y;
+  const int k2 = min((int)bbox[1], half);
+  const int lo = (k2 == half) ? 1 - k2 : -k2, hi = k2;
+  float vmax = 0.f;
+  fipfft::any_load_roots(s_fft, p, tw);
+  for (int rp = blockIdx.x; rp < n / 2; rp += gridDim.x) {
+    const int yy1 = 2 * rp;
+    // Z[c] = X1[c] + i X2[c], X(-c) = conj X(c); self-conjugate bins are real.
+    fipfft::any_stage(s_fft, p, lo, hi, tw, [&](int c) {
+      const int a = c < 0 ? -c : c;
+      const float4 ab = *reinterpret_cast<const float4*>(P + (size_t)a * n + yy1);
+      const bool self = a == 0 || a == half;
+      const float ay = self ? 0.f : ab.y, by = self ? 0.f : ab.w;
+      return c >= 0 ? make_float2(ab.x - by, ay + ab.z) : make_float2(ab.x + by, ab.z - ay);
+    });
+    __syncthreads();
+    const float2* y = fipfft::any_run(s_fft, p, tw);
+    const float ry1 = rck[abs(yy1 - h)], ry2 = rck[abs(yy1 + 1 - h)];
+    float* row1 = pre + (size_t)yy1 * n;
+    float* row2 = row1 + n;
+    for (int o = threadIdx.x; o < n; o += blockDim.x) {
+      const float2 v = fipfft::any_fetch(y, p.m, o);
+      const float rx = rck[abs(o - h)];
+      const float a = fabsf(v.x * (rx * ry1)), b = fabsf(v.y * (rx * ry2));
+      row1[o] = a;
+      row2[o] = b;
+      vmax = fmaxf(vmax, fmaxf(a, b));
+    }
+    __syncthreads();
+  }
+  block_max_to(vmax, &bbox[3]);
+}
+
+// Crop + correction of the cuFFT C2R output (images whose grid side the
+// transforms above do not cover): row (y mod G), column (x mod G), row stride G + 2 floats.
 __global__ void k_correct_c2r(const float* __restrict__ fft_out, const float* __restrict__ ck,
                               int n, int g, float* __restrict__ pre, unsigned* pre_max) {
   const int xx = blockIdx.x * blockDim.x + threadIdx.x, yy = blockIdx.y;
@@ -478,10 +570,59 @@ __global__ void k_correct_c2r(const float* __restrict__ fft_out, const float* __
 
 }  // namespace
 
-bool fip_fft_plan(int g, fipfft::Plan& p, int values_per_thread) {
-  if (g < 48 || g % 3 != 0) return false;
+// Run-time passes for M = G / 3: the largest prime factors first (one pass
+// each above 7), then 7s, and the 2, 3, 5 part in the fewest passes, odd radices
+// first (their first-pass stores fall on distinct banks).
+static bool plan_any(int g, fipfft::Plan& p) {
   const int m = g / 3;
-  if (m & (m - 1)) return false;
+  p = fipfft::Plan{};
+  if (m < 8 || m % 2 != 0) return false;
+  if (((size_t)fipfft::any_roots(m) + kAnyPrime) * sizeof(float2) > (size_t)kAnySmem) return false;
+  int r = m, big[fipfft::kMaxPasses], nbig = 0, e2 = 0, e3 = 0, e5 = 0;
+  while (r % 2 == 0) r /= 2, ++e2;
+  while (r % 3 == 0) r /= 3, ++e3;
+  while (r % 5 == 0) r /= 5, ++e5;
+  for (int f = 7; r > 1; f += 2)
+    while (r % f == 0) {
+      if (f > any_prime_limit(m) || nbig >= 4) return false;
+      big[nbig++] = f;
+      r /= f;
+    }
+  int n = 0;
+  for (int k = nbig - 1; k >= 0; --k) p.radix[n++] = big[k];
+  // Pair the factors into codelets: 15, 9, 10, 12, 6, then powers of two.
+  while (e3 && e5) p.radix[n++] = 15, --e3, --e5;
+  while (e3 >= 2) p.radix[n++] = 9, e3 -= 2;
+  int tail[fipfft::kMaxPasses], nt = 0;
+  while (e5 && n + nt < 10) {
+    if (e2 > 0) tail[nt++] = 10, --e2; else tail[nt++] = 5;
+    --e5;
+  }
+  while (e3 && n + nt < 10) {
+    if (e2 > 1) tail[nt++] = 12, e2 -= 2;
+    else if (e2 == 1) tail[nt++] = 6, --e2;
+    else tail[nt++] = 3;
+    --e3;
+  }
+  while (e2 > 0 && n + nt < fipfft::kMaxPasses) {
+    const int t = e2 >= 4 && e2 != 5 && e2 != 6 ? 4 : (e2 >= 3 ? 3 : e2);
+    tail[nt++] = 1 << t;
+    e2 -= t;
+  }
+  if (e2 || e3 || e5 || n + nt > fipfft::kMaxPasses) return false;
+  for (int k = 0; k < nt; ++k) p.radix[n++] = tail[k];
+  p.g = g;
+  p.m = m;
+  p.any = 1;
+  p.passes = n;
+  p.nt = std::max(64, std::min(kAnyThreads, (3 * m / 8 + 31) / 32 * 32));
+  return true;
+}
+
+bool fip_fft_plan(int g, fipfft::Plan& p, int values_per_thread) {
+  if (g < 24 || g % 3 != 0) return false;
+  const int m = g / 3;
+  if ((m & (m - 1)) || g < 48) return values_per_thread == 0 && plan_any(g, p);
   int lm = 0;
   while ((1 << lm) < m) ++lm;
   // Instantiated: 8 values per thread for M = 2^4..2^11, 16 for 2^5..2^12
@@ -493,6 +634,7 @@ bool fip_fft_plan(int g, fipfft::Plan& p, int values_per_thread) {
   if (values_per_thread == 16) le = 4;
   if (le == 3 && (lm < 4 || lm > 11)) return false;
   if (le == 4 && (lm < 5 || lm > 12)) return false;
+  p = fipfft::Plan{};
   p.g = g;
   p.m = m;
   p.lm = lm;
@@ -642,6 +784,42 @@ static cudaError_t launch_rows(const FipGeom& geo, const float2* colbuf, unsigne
   return cudaGetLastError();
 }
 
+// CTAs of a run-time pass over `items` columns or row pairs.
+static int any_ctas(const void* fn, const fipfft::Plan& plan, size_t smem, int items,
+                    cudaError_t& e) {
+  e = fft_smem_attr(fn, smem);
+  if (e != cudaSuccess) return 0;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, plan.nt, smem);
+  return std::max(1, std::min(items, std::max(1, per_sm) * sm_count()));
+}
+
+static cudaError_t launch_any_cols(const FipGeom& geo, const float2* grid, const unsigned* bbox,
+                                   float2* colbuf, const float2* tw, const fipfft::Plan& plan,
+                                   cudaStream_t s, int batch, size_t grid_stride,
+                                   size_t col_stride) {
+  const size_t smem = (size_t)fipfft::any_smem_elems(plan) * sizeof(float2);
+  cudaError_t e;
+  const int ctas = any_ctas((const void*)k_fft_any_cols, plan, smem, geo.hp, e);
+  if (e != cudaSuccess) return e;
+  k_fft_any_cols<<<dim3(ctas, batch), plan.nt, smem, s>>>(grid, bbox, colbuf, tw, plan,
+                                                          grid_stride, col_stride);
+  return cudaGetLastError();
+}
+
+static cudaError_t launch_any_rows(const FipGeom& geo, const float2* colbuf, unsigned* bbox,
+                                   const float* taper, const float2* tw,
+                                   const fipfft::Plan& plan, float* pre, cudaStream_t s,
+                                   int batch, size_t col_stride, size_t pre_stride) {
+  const size_t smem = (size_t)fipfft::any_smem_elems(plan) * sizeof(float2);
+  cudaError_t e;
+  const int ctas = any_ctas((const void*)k_fft_any_rows, plan, smem, geo.n / 2, e);
+  if (e != cudaSuccess) return e;
+  k_fft_any_rows<<<dim3(ctas, batch), plan.nt, smem, s>>>(
+      colbuf, bbox, taper + geo.n / 2 + 1, pre, tw, plan, col_stride, pre_stride);
+  return cudaGetLastError();
+}
+
 // Calls F<LM, LE> for the plan's instantiation.
 #define FIP_FFT_SWITCH(PLAN, CALL)                                      \
   do {                                                                  \
@@ -672,6 +850,9 @@ cudaError_t fip_launch_fft_cols(const FipGeom& geo, const float2* grid, const un
                                 cudaStream_t s, int batch, size_t grid_stride,
                                 size_t col_stride) {
   if (plan.g != geo.g || batch < 1 || batch > 65535) return cudaErrorInvalidValue;
+  if (plan.any)
+    return launch_any_cols(geo, grid, bbox, colbuf, twiddles, plan, s, batch, grid_stride,
+                           col_stride);
   FIP_FFT_SWITCH(plan, (launch_cols<LM_, LE_>(geo, grid, bbox, colbuf, twiddles, s, batch,
                                               grid_stride, col_stride, plan.split,
                                               plan.direct)));
@@ -682,6 +863,9 @@ cudaError_t fip_launch_fft_rows(const FipGeom& geo, const float2* colbuf, unsign
                                 const fipfft::Plan& plan, float* pre, cudaStream_t s, int batch,
                                 size_t col_stride, size_t pre_stride) {
   if (plan.g != geo.g || batch < 1 || batch > 65535) return cudaErrorInvalidValue;
+  if (plan.any)
+    return launch_any_rows(geo, colbuf, bbox, taper, twiddles, plan, pre, s, batch, col_stride,
+                           pre_stride);
   FIP_FFT_SWITCH(plan, (launch_rows<LM_, LE_>(geo, colbuf, bbox, taper, twiddles, pre, s, batch,
                                               col_stride, pre_stride, plan.split,
                                               plan.direct)));
