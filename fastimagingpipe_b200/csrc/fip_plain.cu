@@ -594,10 +594,16 @@ __device__ __forceinline__ float load_vis(const void* p, int v) {
 // Shared-memory layout of one gridding work item: the tile (int32 fixed
 // point) and the bound reduction; the precision form adds the tile's low
 // limbs.
-constexpr int kTS = FIP_GTILE + 8;  // padded row stride: 4 tap rows x 8 columns hit 32 banks
+// Row stride: odd, so that the commit's walk down a column (the band layout's
+// contiguous direction) reads 32 banks.  (With a stride of 72 that walk hit
+// four banks, 38 % of the gridder's shared-memory wavefronts.)
+constexpr int kTS = FIP_GTILE + 1;
+static_assert(FIP_GTILE * kTS % 4 == 0, "the tile is zeroed in 16-byte stores");
 struct GridSmem {
-  float re[FIP_GTILE * kTS], im[FIP_GTILE * kTS];
   float bound[kThreads / 32];
+  // Real and imaginary sums (plain form, or the high limbs), then the
+  // precision form's low limbs.
+  float tile[2 * FIP_GTILE * kTS];
 };
 // Dynamic shared memory of a gridding CTA.
 __host__ __device__ constexpr size_t grid_smem_bytes(bool comp) {
@@ -653,18 +659,36 @@ __device__ __forceinline__ void entry_taps(const float* __restrict__ B, const vo
   // tile's rows of the footprint are one run of ia along which the tile row
   // moves by +1 (mirrored: -1).
   int ia_lo = 9, ia_hi = 0, lr_first = 0;
-#pragma unroll
-  for (int a = 0; a < 9; ++a)
-    if (a < nr) {
-      const int lr = wrap_row(mir ? -(f.a0 + a) : f.a0 + a, g) - trow0;
-      if ((unsigned)lr < (unsigned)FIP_GTILE) {
-        if (a < ia_lo) {
-          ia_lo = a;
-          lr_first = lr;
-        }
-        ia_hi = a + 1;
-      }
+  if (g >= FIP_GTILE + 9) {
+    // Tile row of ia = 0 before wrapping, or from the other grid end where
+    // that reaches the tile.
+    const int rows = min(FIP_GTILE, g - trow0);  // of the tile
+    const int first = (mir ? -f.a0 : f.a0) - trow0;
+    if (!mir) {
+      const int off = first > -9 && first < rows ? first : first + g;
+      ia_lo = max(0, -off);
+      ia_hi = min(nr, rows - off);
+      lr_first = off + ia_lo;
+    } else {
+      const int off = first >= 0 && first < rows + 9 ? first : first + g;
+      ia_lo = max(0, off - rows + 1);
+      ia_hi = min(nr, off + 1);
+      lr_first = off - ia_lo;
     }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 9; ++a)
+      if (a < nr) {
+        const int lr = wrap_row(mir ? -(f.a0 + a) : f.a0 + a, g) - trow0;
+        if ((unsigned)lr < (unsigned)FIP_GTILE) {
+          if (a < ia_lo) {
+            ia_lo = a;
+            lr_first = lr;
+          }
+          ia_hi = a + 1;
+        }
+      }
+  }
   e.ia_lo = ia_lo;
   e.ia_hi = ia_hi;
   e.ib_lo = max(0, tcol0 - c0);
@@ -672,22 +696,21 @@ __device__ __forceinline__ void entry_taps(const float* __restrict__ B, const vo
   e.cell0 = lr_first * kTS + (c0 + e.ib_lo - tcol0);
   e.r1 = mir ? -(f.a0 + ia_lo) : f.a0 + ia_lo;
   const float ihs = 1 / static_cast<float>(FIP_SUPPORT / 2);
+  // Row taps r1 = a0 + ia; column taps in half-plane order c0 .. c1: original
+  // r2 = c (direct) or -c (mirrored); on the Nyquist column, always a direct
+  // footprint's only one, r2 = -G/2 (r2 never reaches +G/2,
+  // FIPkernels.cu:203).  Integers below 2^24: exact in FP32.  The ninth tap
+  // exists only for a position exactly on a cell.
+  const bool down = mir || 2 * c0 == g;
+  const float r0 = (float)f.a0, q0 = (float)(down ? -c0 : c0), qs = down ? -1.0f : 1.0f;
 #pragma unroll
-  for (int a = 0; a < 9; ++a)
-    e.k1[a] = (a >= ia_lo && a < ia_hi)
-                  ? fipref::es((static_cast<float>(f.a0 + a) - f.p1) * ihs)
-                  : 0.f;
-  // Column taps in half-plane order c0..c1: original r2 = c (direct) or -c
-  // (mirrored); on the Nyquist column a direct tap is r2 = -G/2 (r2 never
-  // reaches +G/2, FIPkernels.cu:203).
-#pragma unroll
-  for (int b = 0; b < 9; ++b) {
-    const int c = c0 + b;
-    const int r2 = mir ? -c : (2 * c == g ? -c : c);
-    e.k2[b] = (b >= e.ib_lo && b < e.ib_hi)
-                  ? fipref::es((static_cast<float>(r2) - f.p2) * ihs)
-                  : 0.f;
+  for (int k = 0; k < 8; ++k) {
+    e.k1[k] = fipref::es(((r0 + (float)k) - f.p1) * ihs);
+    e.k2[k] = fipref::es(((q0 + qs * (float)k) - f.p2) * ihs);
   }
+  e.k1[8] = e.k2[8] = 0.f;
+  if (nr > 8) e.k1[8] = fipref::es(((r0 + 8.0f) - f.p1) * ihs);
+  if (nc > 8) e.k2[8] = fipref::es(((q0 + qs * 8.0f) - f.p2) * ihs);
 }
 
 // One gridding work item (tile, entry range) of one snapshot, a thread per
@@ -718,13 +741,11 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tile = item.x, cnt = item.z - item.y;
   const int trow0 = (tile / tiles_c) * FIP_GTILE, tcol0 = (tile % tiles_c) * FIP_GTILE;
-  for (int k = threadIdx.x; k < FIP_GTILE * kTS; k += kThreads) {
-    S.re[k] = 0.f;
-    S.im[k] = 0.f;
-    if (COMP) {
-      s_cre[k] = 0.f;
-      s_cim[k] = 0.f;
-    }
+  // The tile (and, behind it, its low limbs) zeroed in 16-byte stores.
+  {
+    constexpr int kWords = (2 + (COMP ? 2 : 0)) * FIP_GTILE * kTS / 4;
+    for (int k = threadIdx.x; k < kWords; k += kThreads)
+      reinterpret_cast<float4*>(S.tile)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   // Phase 1: this thread's entry.
   const int q = threadIdx.x;
@@ -753,8 +774,8 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
     fx = ldexpf(1.0f, 45 - ex);
     fx_inv = ldexpf(1.0f, ex - 45);
   }
-  int* s_qre = reinterpret_cast<int*>(S.re);
-  int* s_qim = reinterpret_cast<int*>(S.im);
+  int* s_qre = reinterpret_cast<int*>(S.tile);
+  int* s_qim = s_qre + FIP_GTILE * kTS;
   unsigned* s_lre = reinterpret_cast<unsigned*>(s_cre);
   unsigned* s_lim = reinterpret_cast<unsigned*>(s_cim);
   // Exact limbs of t = x * 2^e (precision form, see above).
@@ -769,60 +790,81 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
   if (have && !et.empty()) {
     const float wrf = COMP ? et.wr : et.wr * fx, wif = COMP ? et.wi : et.wi * fx;
     const int dstep = et.mir ? -kTS : kTS;
-    const int lc0 = et.cell0 - (wrap_row(et.r1, g) - trow0) * kTS;
+    const unsigned rn = et.ia_hi - et.ia_lo, cn = et.ib_hi - et.ib_lo;
+    const int cell = et.cell0 - et.ib_lo;  // of tap (ia_lo, 0)
+    auto add = [&](int c, float x, float y) {
+      if (!COMP) {
+        atomicAdd(&s_qre[c], __float2int_rn(x));
+        atomicAdd(&s_qim[c], __float2int_rn(y));
+      } else {
+        int hr, hi;
+        unsigned lr2, li2;
+        limbs(x, hr, lr2);
+        limbs(y, hi, li2);
+        atomicAdd(&s_qre[c], hr);
+        atomicAdd(&s_lre[c], lr2);
+        atomicAdd(&s_qim[c], hi);
+        atomicAdd(&s_lim[c], li2);
+      }
+    };
+    if (g >= FIP_GTILE + 9) {
+      int rc = cell - et.ia_lo * dstep;
 #pragma unroll
-    for (int a = 0; a < 9; ++a) {
-      if (a < et.ia_lo || a >= et.ia_hi) continue;
+      for (int a = 0; a < 8; ++a, rc += dstep) {
+        if ((unsigned)(a - et.ia_lo) >= rn) continue;
+        const float ra = wrf * et.k1[a], rb = wif * et.k1[a];
+#pragma unroll
+        for (int b = 0; b < 8; ++b)
+          if ((unsigned)(b - et.ib_lo) < cn) add(rc + b, ra * et.k2[b], rb * et.k2[b]);
+        if (et.ib_hi > 8) add(rc + 8, ra * et.k2[8], rb * et.k2[8]);
+      }
+      if (et.ia_hi > 8) {
+        const float ra = wrf * et.k1[8], rb = wif * et.k1[8];
+#pragma unroll
+        for (int b = 0; b < 9; ++b)
+          if ((unsigned)(b - et.ib_lo) < cn) add(rc + b, ra * et.k2[b], rb * et.k2[b]);
+      }
+    } else {
       // Grids of little more than one tile: a tile may hold rows from both
       // grid ends, with the rows between them in another tile or none, so
       // each tap row is wrapped and checked on its own.
-      int rc = et.cell0 + (a - et.ia_lo) * dstep;
-      if (g < FIP_GTILE + 9) {
+      const int lc0 = cell - (wrap_row(et.r1, g) - trow0) * kTS;
+#pragma unroll
+      for (int a = 0; a < 9; ++a) {
+        if ((unsigned)(a - et.ia_lo) >= rn) continue;
         const int lr = wrap_row(et.r1 + (et.mir ? et.ia_lo - a : a - et.ia_lo), g) - trow0;
         if ((unsigned)lr >= (unsigned)FIP_GTILE) continue;
-        rc = lr * kTS + lc0;
-      }
-      const float ra = wrf * et.k1[a], rb = wif * et.k1[a];
+        const float ra = wrf * et.k1[a], rb = wif * et.k1[a];
 #pragma unroll
-      for (int b = 0; b < 9; ++b) {
-        if (b < et.ib_lo || b >= et.ib_hi) continue;
-        const int c = rc + (b - et.ib_lo);
-        if (!COMP) {
-          atomicAdd(&s_qre[c], __float2int_rn(ra * et.k2[b]));
-          atomicAdd(&s_qim[c], __float2int_rn(rb * et.k2[b]));
-        } else {
-          int hr, hi;
-          unsigned lr2, li2;
-          limbs(ra * et.k2[b], hr, lr2);
-          limbs(rb * et.k2[b], hi, li2);
-          atomicAdd(&s_qre[c], hr);
-          atomicAdd(&s_lre[c], lr2);
-          atomicAdd(&s_qim[c], hi);
-          atomicAdd(&s_lim[c], li2);
-        }
+        for (int b = 0; b < 9; ++b)
+          if ((unsigned)(b - et.ib_lo) < cn)
+            add(lr * kTS + lc0 + b, ra * et.k2[b], rb * et.k2[b]);
       }
     }
   }
   __syncthreads();
-  // Phase 3: commit in the layout's contiguous direction.
+  // Phase 3: commit in the layout's contiguous direction: each thread keeps its
+  // place along it and steps across.
   const bool single = item.w != 0;
-  for (int k = threadIdx.x; k < FIP_GTILE * FIP_GTILE; k += kThreads) {
-    const int lr = layout ? k % FIP_GTILE : k / FIP_GTILE;
-    const int lc = layout ? k / FIP_GTILE : k % FIP_GTILE;
-    const int row = trow0 + lr, col = tcol0 + lc;
-    if (row < g && col < hp) {
+  const int along = threadIdx.x % FIP_GTILE, across0 = threadIdx.x / FIP_GTILE;
+  constexpr int kStep = kThreads / FIP_GTILE;
+  const int na = layout ? g - trow0 : hp - tcol0, nx = layout ? hp - tcol0 : g - trow0;
+  const int sa = layout ? kTS : 1, sx = layout ? 1 : kTS;  // shared strides along, across
+  float2* dst = grid + cell_index(trow0, tcol0, g, hp, layout) + along +
+                (size_t)across0 * (layout ? g : hp);
+  const size_t dstep = (size_t)kStep * (layout ? g : hp);
+  int at = along * sa + across0 * sx;
+  if (along < na) {
+#pragma unroll 4
+    for (int k = 0; k < FIP_GTILE / kStep; ++k, at += kStep * sx, dst += dstep) {
+      if (across0 + k * kStep >= nx) break;
       float2 val;
       if (COMP) {
-        const int at = lr * kTS + lc;
-        const unsigned* s_lre = reinterpret_cast<const unsigned*>(s_cre);
-        const unsigned* s_lim = reinterpret_cast<const unsigned*>(s_cim);
         val = make_float2((float)(((double)s_qre[at] * 8388608.0 + (double)s_lre[at]) * fx_inv),
                           (float)(((double)s_qim[at] * 8388608.0 + (double)s_lim[at]) * fx_inv));
       } else {
-        val = make_float2((float)s_qre[lr * kTS + lc] * fx_inv,
-                          (float)s_qim[lr * kTS + lc] * fx_inv);
+        val = make_float2((float)s_qre[at] * fx_inv, (float)s_qim[at] * fx_inv);
       }
-      float2* dst = &grid[cell_index(row, col, g, hp, layout)];
       if (single) {
         *dst = val;
       } else if (val.x != 0.f || val.y != 0.f) {
