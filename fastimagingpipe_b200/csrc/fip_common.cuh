@@ -15,7 +15,13 @@
 
 // Grid tiles used by the binned gridder (cells of the half-plane grid).
 #define FIP_GTILE 64
-#define FIP_GCHUNK 256  // virtual visibilities per gridding work item
+#define FIP_GCHUNK 256  // virtual visibilities per gridding work item, by default
+// ... and at most: a work item's low limbs (precision form) sum up to 2^23 per
+// entry in 32 bits.
+#define FIP_GCHUNK_MAX 480
+// Work items a binning of adaptive chunks may need beyond one per tile and one
+// per FIP_GCHUNK entries (fip_grid_chunk).
+#define FIP_GITEMS_SPARE 3072
 
 // Geometry of one image size.  The uv grid is the Hermitian half plane
 // G x (G/2+1) complex (row stride hp = G/2+1 complex = G+2 floats), which is
@@ -106,6 +112,7 @@ struct FipBinSnap {
   float scale;     // cell * G
   int g, hp, tiles_c, ntiles, layout;
   unsigned wcap;
+  unsigned chunk;  // entries per work item
   unsigned* count;
   unsigned* offset;
   unsigned* cursor;

@@ -547,7 +547,7 @@ int fip_imager_create(fip_imager** out, const fip_imager_config* cfg) {
     FIP_ALLOC(cudaEventCreateWithFlags(&L.ev_done, cudaEventDisableTiming));
     FIP_ALLOC(cudaEventCreateWithFlags(&L.ev_targets, cudaEventDisableTiming));
     L.bins.cap = 12 * nb;
-    L.bins.wcap = ntiles + L.bins.cap / FIP_GCHUNK + 1;
+    L.bins.wcap = ntiles + L.bins.cap / FIP_GCHUNK + FIP_GITEMS_SPARE;
   }
   // Every lane's `member`, `count` elements each, from one allocation.
 #define FIP_LANES(member, count)                                            \
@@ -2034,7 +2034,7 @@ int seq_alloc(BatchSeq& q, size_t smax, size_t& tot) {
   const size_t S = smax, nb = cfg.max_baselines;
   q.ntiles = (size_t)geo.tiles_r * geo.tiles_c;
   q.cap = 12 * nb;
-  q.wcap = q.ntiles + q.cap / FIP_GCHUNK + 1;
+  q.wcap = q.ntiles + q.cap / FIP_GCHUNK + FIP_GITEMS_SPARE;
   q.n2 = (size_t)geo.n * geo.n;
   q.grid_elems = (size_t)geo.g * geo.hp;
   q.col_elems = (size_t)geo.hp * geo.n;

@@ -51,6 +51,8 @@ cudaError_t fip_launch_bin_batch(FipBinBatch& in, unsigned* base, cudaStream_t s
 // CTAs per snapshot of a binning launch over `count` snapshots of up to
 // nbmax visibilities; ctas * count <= kFipBinCtas.
 constexpr int kFipBinCtas = 296;
+// Entries per gridding work item of a launch over `nb` visibilities in all.
+unsigned fip_grid_chunk(size_t nb);
 int fip_bin_ctas(int count, size_t nbmax);
 // Kernels fip_launch_bin launches for nb > 0.
 int fip_bin_launches(const FipGeom& geo);

@@ -28,6 +28,7 @@ constexpr size_t kMaxImage = 4096;
 constexpr int kMaxTiles = 96 * 49;
 constexpr size_t kMaxEntries = 12 * kMaxBaselines;  // <= 12 tile entries per visibility
 constexpr size_t kMaxWork = kMaxTiles + kMaxEntries / FIP_GCHUNK + 1;
+static_assert(kMaxEntries / FIP_GCHUNK >= FIP_GITEMS_SPARE, "adaptive chunks' items");
 
 // Layout of the scratch: the per-tile bins of one snapshot.
 struct Scratch {

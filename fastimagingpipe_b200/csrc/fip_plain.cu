@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(kScanThreads) k_bin_scan_tiles(
   extern __shared__ unsigned s_wp[];  // [ntiles] first work item of each split tile
   const FipBinSnap& sn = in.s[blockIdx.x];
   const int ntiles = sn.ntiles, tiles_c = sn.tiles_c, g = sn.g;
-  const unsigned wcap = sn.wcap;
+  const unsigned wcap = sn.wcap, chunk = sn.chunk;
   const int k1 = (int)sn.bbox[0], k2 = (int)sn.bbox[1];
   const bool full = sn.layout == 0;
   uint3 carry = make_uint3(0, 0, 0);
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(kScanThreads) k_bin_scan_tiles(
     for (int k = 0; k < kScanPer; ++k) {
       const int r0 = tr * FIP_GTILE, r1 = min(r0 + FIP_GTILE, g) - 1;
       const bool band = full || (tc * FIP_GTILE <= k2 && (r0 <= k1 || r1 >= g - k1));
-      nch[k] = t0 + k < ntiles && band ? max(1u, (c[k] + FIP_GCHUNK - 1) / FIP_GCHUNK) : 0u;
+      nch[k] = t0 + k < ntiles && band ? max(1u, (c[k] + chunk - 1) / chunk) : 0u;
       if (++tc == tiles_c) {
         tc = 0;
         ++tr;
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(kScanThreads) k_bin_scan_tiles(
         sn.offset[t] = run;
         if (!sn.base) sn.cursor[t] = 0;
         if (nch[k] > 0 && wrun < wcap)
-          sn.work[wrun] = make_int4(t, (int)run, (int)(run + min((unsigned)FIP_GCHUNK, c[k])),
+          sn.work[wrun] = make_int4(t, (int)run, (int)(run + min(chunk, c[k])),
                                     nch[k] == 1);
         if (nch[k] > 1) {
           sn.multi[mrun++] = (unsigned)t;
@@ -509,11 +509,11 @@ __global__ void __launch_bounds__(kScanThreads) k_bin_scan_tiles(
   __syncthreads();
   for (unsigned m = threadIdx.x >> 5; m < carry.z; m += kScanThreads / 32) {
     const unsigned t = sn.multi[m], run = sn.offset[t], c = sn.count[t], w0 = s_wp[t];
-    const unsigned n = (c + FIP_GCHUNK - 1) / FIP_GCHUNK;
+    const unsigned n = (c + chunk - 1) / chunk;
     for (unsigned q = 1 + (threadIdx.x & 31); q < n; q += 32)
       if (w0 + q < wcap)
-        sn.work[w0 + q] = make_int4((int)t, (int)(run + q * FIP_GCHUNK),
-                                    (int)(run + min((q + 1) * FIP_GCHUNK, c)), 0);
+        sn.work[w0 + q] = make_int4((int)t, (int)(run + q * chunk),
+                                    (int)(run + min((q + 1) * chunk, c)), 0);
   }
 }
 
@@ -610,29 +610,13 @@ __host__ __device__ constexpr size_t grid_smem_bytes(bool comp) {
   return sizeof(GridSmem) + (comp ? 2 * FIP_GTILE * kTS * sizeof(float) : 0);
 }
 
-// One entry's taps inside a tile: its weights (halved for the Hermitian
-// split, conjugated for the mirrored copy), its in-tile rows ia in [ia_lo,
-// ia_hi) and columns ib in [ib_lo, ib_hi) of the footprint, the tile cell
-// cell0 of tap (ia_lo, ib_lo), the row direction and the separable kernel
-// values of the in-tile rows and columns.
-struct EntryTaps {
-  float wr, wi;
-  int ia_lo, ia_hi, ib_lo, ib_hi, cell0, r1, mir;
-  float k1[9], k2[9];
-  __device__ bool empty() const { return ia_lo >= ia_hi || ib_lo >= ib_hi; }
-};
-
+// Weights of one entry: the visibility (FIPkernels.cu:188-195), halved for the
+// Hermitian split, conjugated for the mirrored copy.
 template <int VT>
-__device__ __forceinline__ void entry_taps(const float* __restrict__ B, const void* vr,
-                                           const void* vi, const float* vis_scale, float inten,
-                                           float scale, int g, unsigned ent, int trow0,
-                                           int tcol0, const FipRawVis& raw, EntryTaps& e) {
+__device__ __forceinline__ void entry_weights(const void* vr, const void* vi,
+                                              const float* vis_scale, float inten, unsigned ent,
+                                              const FipRawVis& raw, float& owr, float& owi) {
   const int v = (int)(ent >> 1), mir = (int)(ent & 1);
-  Footprint f;
-  footprint(B[2 * v], B[2 * v + 1], scale, g, f);
-  int c0, c1;
-  half_cols(f, mir, g, c0, c1);
-  // Visibility weighting (FIPkernels.cu:188-195).
   float wr, wi;
   if constexpr (VT == FIP_VIS_RAW) {
     // Stokes-I collapse fused into the load: no collapsed copy in memory.
@@ -649,8 +633,26 @@ __device__ __forceinline__ void entry_taps(const float* __restrict__ B, const vo
     wr = (load_vis<VT>(vr, v) * sc) / inten;
     wi = (load_vis<VT>(vi, v) * sc) / inten;
   }
-  e.wr = 0.5f * wr;
-  e.wi = mir ? -0.5f * wi : 0.5f * wi;
+  owr = 0.5f * wr;
+  owi = mir ? -0.5f * wi : 0.5f * wi;
+}
+
+// One entry's taps inside a tile: its in-tile rows ia in [ia_lo, ia_hi) and
+// columns ib in [ib_lo, ib_hi) of the footprint, the tile cell cell0 of tap
+// (ia_lo, ib_lo), the row direction and the separable kernel values.
+struct EntryTaps {
+  int ia_lo, ia_hi, ib_lo, ib_hi, cell0, r1, mir;
+  float k1[9], k2[9];
+  __device__ bool empty() const { return ia_lo >= ia_hi || ib_lo >= ib_hi; }
+};
+
+__device__ __forceinline__ void entry_taps(const float* __restrict__ B, float scale, int g,
+                                           unsigned ent, int trow0, int tcol0, EntryTaps& e) {
+  const int v = (int)(ent >> 1), mir = (int)(ent & 1);
+  Footprint f;
+  footprint(B[2 * v], B[2 * v + 1], scale, g, f);
+  int c0, c1;
+  half_cols(f, mir, g, c0, c1);
   e.mir = mir;
   const int nr = f.a1 - f.a0 + 1, nc = c1 - c0 + 1;
   // Tap row ia is grid row wrap(r1), r1 = a0 + ia (mirrored: -(a0 + ia)).
@@ -713,19 +715,18 @@ __device__ __forceinline__ void entry_taps(const float* __restrict__ B, const vo
   if (nc > 8) e.k2[8] = fipref::es(((q0 + qs * 8.0f) - f.p2) * ihs);
 }
 
-// One gridding work item (tile, entry range) of one snapshot, a thread per
-// entry (at most one per thread: FIP_GCHUNK <= kThreads).  Phase 1 takes the
-// thread's entry footprint and kernel values into registers and reduces the
-// item's bound, phase 2 walks the entry's in-tile taps into the shared
-// tile, phase 3 commits.  The tile sums are fixed point, so the shared-memory
+// One gridding work item (tile, entry range) of one snapshot, one or two
+// entries per thread.  Phase 1 loads their weights and reduces the item's
+// bound, phase 2 takes an entry's footprint and kernel values into registers
+// and walks its in-tile taps into the shared tile, phase 3 commits.  The tile sums are fixed point, so the shared-memory
 // sums are native integer atomics: exact and independent of their order.
-// Plain form: q = round(tap * 2^30 / bound) in one int32, `bound` (the
+// Plain form: q = round(tap * 2^31 / bound) in one int32, `bound` (the
 // item's summed weights) bounding every cell sum.
 // Precision form with FP32 visibilities (COMP; with FP16/BF16 storage the
 // precision form sums as the plain form does): t = tap * 2^e, 2^e = the power of two with
 // bound * 2^e < 2^45, is exact in FP32 and is split exactly into
 // hi * 2^23 + lo (hi < 2^22 in magnitude, 0 <= lo <= 2^23), two int32 limbs
-// summed separately (at most 256 taps per cell per item: no overflow), so a
+// summed separately (FIP_GCHUNK_MAX taps per cell per item at most: no overflow), so a
 // cell holds the exact sum of its FP32 taps to 2^-45 of the bound and is
 // rounded once at the commit.
 template <int VT, bool COMP>
@@ -737,7 +738,7 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
                                           int layout, const unsigned* __restrict__ entries,
                                           int4 item, float2* __restrict__ grid,
                                           const FipRawVis& raw = FipRawVis{}) {
-  static_assert(FIP_GCHUNK <= kThreads, "one entry per thread at most");
+  static_assert(FIP_GCHUNK_MAX <= 2 * kThreads, "two entries per thread at most");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tile = item.x, cnt = item.z - item.y;
   const int trow0 = (tile / tiles_c) * FIP_GTILE, tcol0 = (tile % tiles_c) * FIP_GTILE;
@@ -747,16 +748,19 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
     for (int k = threadIdx.x; k < kWords; k += kThreads)
       reinterpret_cast<float4*>(S.tile)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  // Phase 1: this thread's entry.
-  const int q = threadIdx.x;
-  const bool have = q < cnt;
-  EntryTaps et;
-  float bound = 0.f;  // sum over the item of max(|wr|, |wi|): bounds every cell sum
+  // Phase 1: the weights of this thread's entries (one, or two in items of
+  // more than kThreads).
+  const bool have = (int)threadIdx.x < cnt, more = (int)threadIdx.x + kThreads < cnt;
+  unsigned ent = 0, ent2 = 0;
+  float wr = 0.f, wi = 0.f, wr2 = 0.f, wi2 = 0.f;
   if (have) {
-    entry_taps<VT>(B, vr, vi, vis_scale, inten, scale, g, entries[item.y + q], trow0, tcol0,
-                   raw, et);
-    bound = fmaxf(fabsf(et.wr), fabsf(et.wi));
+    ent = entries[item.y + threadIdx.x];
+    if (more) ent2 = entries[item.y + threadIdx.x + kThreads];
+    entry_weights<VT>(vr, vi, vis_scale, inten, ent, raw, wr, wi);
+    if (more) entry_weights<VT>(vr, vi, vis_scale, inten, ent2, raw, wr2, wi2);
   }
+  // Sum over the item of max(|wr|, |wi|): bounds every cell sum.
+  float bound = fmaxf(fabsf(wr), fabsf(wi)) + fmaxf(fabsf(wr2), fabsf(wi2));
   for (int o = 16; o > 0; o >>= 1) bound += __shfl_xor_sync(0xffffffffu, bound, o);
   if (lane == 0) S.bound[warp] = bound;
   __syncthreads();
@@ -766,8 +770,8 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
   tot *= 1.0001f;  // margin for the rounding of the weights and their sum
   float fx = 0.f, fx_inv = 0.f;
   if (!COMP) {
-    fx = tot > 0.f ? 1073741824.0f / tot : 0.f;
-    fx_inv = tot * (1.0f / 1073741824.0f);
+    fx = tot > 0.f ? 2147483648.0f / tot : 0.f;
+    fx_inv = tot * (1.0f / 2147483648.0f);
   } else if (tot > 0.f) {
     int ex = 0;
     frexpf(tot, &ex);  // tot < 2^ex
@@ -786,9 +790,13 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
     hi = __float_as_int(hf + 12582912.0f) - 0x4B400000;  // |hf| < 2^22: exact
     lo = __float_as_uint(lf + 8388608.0f) - 0x4B000000u;  // round to integer
   };
-  // Phase 2: the thread walks its entry's in-tile taps.
-  if (have && !et.empty()) {
-    const float wrf = COMP ? et.wr : et.wr * fx, wif = COMP ? et.wi : et.wi * fx;
+  // Phase 2: the thread walks its entries' in-tile taps.
+#pragma unroll 1
+  for (int left = have ? (more ? 2 : 1) : 0; left > 0; --left, ent = ent2, wr = wr2, wi = wi2) {
+    EntryTaps et;
+    entry_taps(B, scale, g, ent, trow0, tcol0, et);
+    if (et.empty()) continue;
+    const float wrf = COMP ? wr : wr * fx, wif = COMP ? wi : wi * fx;
     const int dstep = et.mir ? -kTS : kTS;
     const unsigned rn = et.ia_hi - et.ia_lo, cn = et.ib_hi - et.ib_lo;
     const int cell = et.cell0 - et.ib_lo;  // of tap (ia_lo, 0)
@@ -913,13 +921,19 @@ __global__ void __launch_bounds__(kThreads) k_grid_batch(const __grid_constant__
   GridSmem& S = *reinterpret_cast<GridSmem*>(s_raw);
   float* s_cre = reinterpret_cast<float*>(reinterpret_cast<char*>(s_raw) + sizeof(GridSmem));
   float* s_cim = s_cre + FIP_GTILE * kTS;
-  if (threadIdx.x == 0) {
-    unsigned acc = 0;
-    for (int k = 0; k < in.count; ++k) {
-      s_first[k] = acc;
-      acc += *in.s[k].nwork;
+  // (Two snapshots per lane of the first warp.)
+  if (threadIdx.x < 32) {
+    const int k = 2 * threadIdx.x;
+    const unsigned a = k < in.count ? *in.s[k].nwork : 0u;
+    const unsigned b = k + 1 < in.count ? *in.s[k + 1].nwork : 0u;
+    unsigned inc = a + b;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+      if ((int)threadIdx.x >= o) inc += y;
     }
-    s_first[in.count] = acc;
+    if (k <= in.count) s_first[k] = inc - a - b;
+    if (k + 1 <= in.count) s_first[k + 1] = inc - b;
+    if (k + 2 == FIP_MAX_BATCH && in.count == FIP_MAX_BATCH) s_first[FIP_MAX_BATCH] = inc;
   }
   __syncthreads();
   const unsigned total = s_first[in.count];
@@ -1720,6 +1734,16 @@ bool fip_bin_batchable(const FipGeom& geo) {
 
 int fip_bin_launches(const FipGeom& geo) { return fip_bin_batchable(geo) ? 3 : 4; }
 
+// An item's fixed cost (zeroing and committing its tile) asks for large chunks,
+// a launch with few items for enough of them to fill the device: two per SM,
+// about 1.4 entries per visibility.  Two, four and eight items per SM wanted,
+// us: three-snapshot calls at 4096^2 929 / 940 / 951 (plain), 568 / 578 / 590
+// (FP16), at 512^2 72 / 76 / 76; chunks of 256 throughout: 943, 590, 76.
+unsigned fip_grid_chunk(size_t nb) {
+  const size_t want = (size_t)(1.4 * (double)nb) / (2 * 148);
+  return (unsigned)std::max<size_t>(64, std::min<size_t>(FIP_GCHUNK_MAX, want / 32 * 32));
+}
+
 int fip_bin_ctas(int count, size_t nbmax) {
   const size_t per = (size_t)kBinThreads;
   return std::max(1, (int)std::min<size_t>(kFipBinCtas / std::max(1, count),
@@ -1755,14 +1779,19 @@ FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBin
 cudaError_t fip_launch_bin_batch(FipBinBatch& in, unsigned* base, cudaStream_t s) {
   if (in.count < 1 || in.count > FIP_MAX_BATCH) return cudaErrorInvalidValue;
   int ntiles = 0, nb = 0;
+  size_t total = 0;
   for (int k = 0; k < in.count; ++k) {
     ntiles = std::max(ntiles, in.s[k].ntiles);
     nb = std::max(nb, in.s[k].nb);
+    total += (size_t)in.s[k].nb;
   }
   if (ntiles > kMaxSmemTiles) return cudaErrorInvalidValue;
   const int ctas = fip_bin_ctas(in.count, (size_t)nb);
-  for (int k = 0; k < in.count; ++k)
+  const unsigned chunk = fip_grid_chunk(total);
+  for (int k = 0; k < in.count; ++k) {
+    in.s[k].chunk = chunk;
     in.s[k].base = base ? base + (size_t)k * ctas * ntiles : nullptr;
+  }
   const size_t smem = (size_t)ntiles * sizeof(unsigned);
   const dim3 grid(ctas, in.count);
   k_bin_count<<<grid, kBinThreads, smem, s>>>(in);
