@@ -114,11 +114,7 @@ namespace {
 // snapshot, and calls often follow one another) before they block.
 class CopyPool {
  public:
-  struct Seg {
-    void* dst;
-    const void* src;
-    size_t bytes;
-  };
+  using Seg = FipCopySeg;
   static CopyPool& get() {
     static CopyPool pool;
     return pool;
@@ -236,6 +232,8 @@ class CopyPool {
   std::atomic<bool> stop_{false};
 };
 }  // namespace
+
+void fip_host_copy(const FipCopySeg* segs, int count) { CopyPool::get().copy(segs, count); }
 
 // Twiddle tables of the band-pruned transform of length g = 3 M: w^k,
 // w = e^{+2 pi i / g}, for k < g, then the passes' half table W^m = w^{3 m},
@@ -1690,7 +1688,23 @@ struct fip_batch {
   double phase_ms[kPhases] = {};
   long phase_calls = 0;
   bool phase_pending = false;
-  cudaGraphExec_t exec = nullptr;
+  // Executable graphs of the latest call shapes (snapshots per sequence and
+  // their triggers): a call of a known shape updates its graph in place, so
+  // calls that alternate between shapes, as a server's steps do, do not
+  // instantiate anew (0.3 to 0.5 ms each).  At most kMaxExecs, the least
+  // recently used replaced.
+  static constexpr size_t kMaxExecs = 8;
+  struct Exec {
+    std::vector<int> shape;
+    cudaGraphExec_t exec = nullptr;
+    unsigned long long used = 0;
+  };
+  std::vector<Exec> execs;
+  unsigned long long exec_tick = 0;
+  void drop_execs() {
+    for (Exec& e : execs) cudaGraphExecDestroy(e.exec);
+    execs.clear();
+  }
   unsigned long long launches = 0;
 };
 
@@ -1698,7 +1712,7 @@ namespace {
 void batch_free(fip_batch* b) {
   if (!b) return;
   DeviceGuard g(b->cfg.device);
-  if (b->exec) cudaGraphExecDestroy(b->exec);
+  b->drop_execs();
   for (BatchSeq& q : b->seq) q.free_all();
   if (b->theta_tab) cudaFree(b->theta_tab);
   if (b->bin_base) cudaFree(b->bin_base);
@@ -2190,10 +2204,8 @@ int fip_batch_set_profiling(fip_batch* b, int enable) {
   FIP_TRY(batch_collect(b));
   if (enable && !b->phase_ev[0])
     for (cudaEvent_t& e : b->phase_ev) FIP_CUDA(cudaEventCreate(&e));
-  if ((enable != 0) != b->profiling && b->exec) {
-    cudaGraphExecDestroy(b->exec);  // the graph gains or loses its event nodes
-    b->exec = nullptr;
-  }
+  // The graphs gain or lose their event nodes.
+  if ((enable != 0) != b->profiling) b->drop_execs();
   b->profiling = enable != 0;
   for (double& v : b->phase_ms) v = 0.0;
   b->phase_calls = 0;
@@ -2351,29 +2363,51 @@ static int batch_run(fip_batch* b, const int* seq_of, const float* const* vis_re
       FIP_CUDA(cudaGraphKernelNodeSetAttribute(nd, cudaLaunchAttributePriority, &v));
     }
   }
-  // Re-use the executable graph when the call's shape is unchanged (only
-  // pointers, sizes and launch extents differ); instantiate otherwise.
-  bool updated = false;
-  if (b->exec) {
+  // Re-use the executable graph of the call's shape (only pointers, sizes and
+  // launch extents differ); instantiate otherwise.
+  std::vector<int> shape(per, per + nseq);
+  if (slots) {
+    int triggers = 0;
+    for (size_t k = 0; k < count; ++k) triggers += slots[k].prev_image[0] != nullptr;
+    shape.push_back(-1 - triggers);
+  } else {
+    shape.insert(shape.end(), ntrig, ntrig + nseq);
+  }
+  fip_batch::Exec* ex = nullptr;
+  for (fip_batch::Exec& x : b->execs)
+    if (x.shape == shape) ex = &x;
+  if (ex) {
     cudaGraphExecUpdateResultInfo info{};
-    updated = cudaGraphExecUpdate(b->exec, graph, &info) == cudaSuccess;
-    if (!updated) {
+    if (cudaGraphExecUpdate(ex->exec, graph, &info) != cudaSuccess) {
       cudaGetLastError();
-      cudaGraphExecDestroy(b->exec);
-      b->exec = nullptr;
+      cudaGraphExecDestroy(ex->exec);
+      b->execs.erase(b->execs.begin() + (ex - b->execs.data()));
+      ex = nullptr;
     }
   }
-  if (!updated) {
+  if (!ex) {
+    if (b->execs.size() >= fip_batch::kMaxExecs) {
+      auto old = std::min_element(b->execs.begin(), b->execs.end(),
+                                  [](const fip_batch::Exec& x, const fip_batch::Exec& y) {
+                                    return x.used < y.used;
+                                  });
+      cudaGraphExecDestroy(old->exec);
+      b->execs.erase(old);
+    }
     // Per-node priorities (set above) apply only with this flag.
-    e = cudaGraphInstantiate(&b->exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+    fip_batch::Exec fresh;
+    e = cudaGraphInstantiate(&fresh.exec, graph, cudaGraphInstantiateFlagUseNodePriority);
     if (e != cudaSuccess) {
       cudaGraphDestroy(graph);
-      b->exec = nullptr;
       return fail(FIP_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
     }
+    fresh.shape = shape;
+    b->execs.push_back(fresh);
+    ex = &b->execs.back();
   }
+  ex->used = ++b->exec_tick;
   cudaGraphDestroy(graph);
-  FIP_CUDA(cudaGraphLaunch(b->exec, cs));
+  FIP_CUDA(cudaGraphLaunch(ex->exec, cs));
   b->phase_pending = b->profiling;
   if (cs != s) {
     FIP_CUDA(cudaEventRecord(b->fork, cs));
@@ -2490,10 +2524,7 @@ static int batch_autotune(fip_batch* b, const int* seq_of, const float* const* v
     b->grid_ctas_per_sm = chosen;
   }
   // The shapes changed: the next call instantiates a new graph.
-  if (b->exec) {
-    cudaGraphExecDestroy(b->exec);
-    b->exec = nullptr;
-  }
+  b->drop_execs();
   for (BatchSeq& q : b->seq) q.carried = 0;
   return FIP_OK;
 }

@@ -14,6 +14,14 @@
 // Records the calling thread's last error message and returns `code`.
 int fip_set_error(int code, const std::string& msg);
 
+// Host copies of several megabytes, shared by a small pool of threads.
+struct FipCopySeg {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+void fip_host_copy(const FipCopySeg* segs, int count);
+
 // Scratch of the tile-binned gridder for one image size.
 struct FipBins {
   unsigned* count;    // [ntiles] entries per grid tile
@@ -50,7 +58,7 @@ FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBin
 cudaError_t fip_launch_bin_batch(FipBinBatch& in, unsigned* base, cudaStream_t s);
 // CTAs per snapshot of a binning launch over `count` snapshots of up to
 // nbmax visibilities; ctas * count <= kFipBinCtas.
-constexpr int kFipBinCtas = 296;
+constexpr int kFipBinCtas = 592;
 // Entries per gridding work item of a launch over `nb` visibilities in all.
 unsigned fip_grid_chunk(size_t nb);
 int fip_bin_ctas(int count, size_t nbmax);
