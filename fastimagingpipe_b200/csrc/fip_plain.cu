@@ -297,10 +297,10 @@ __global__ void __launch_bounds__(kScanThreads) k_bin_scan(
 // lanes first), and adds its non-zero counts to the global ones, which
 // returns where its entries start within each tile's list; one CTA per
 // snapshot then scans the tiles; the scatter pass starts its shared-memory
-// cursors from the two and fills the lists in one sweep.  Two CTAs per SM
-// over the whole launch: more of them multiply the histograms' fixed cost
-// (zeroing and merging every tile's counter), fewer leave the loads' latency
-// exposed.
+// cursors from the two and fills the lists in one sweep.  A few CTAs per SM
+// over the whole launch (fip_bin_ctas): more of them multiply the histograms'
+// fixed cost (zeroing and merging every tile's counter), fewer leave the
+// loads' latency exposed.
 // Bound: the entries' integer arithmetic, then latency (three dependent
 // launches).  1.05 M visibilities at 2048^2: 25 + 11 + 50 us (count, scan,
 // scatter) with a recount in the scatter pass, 1,184 small CTAs and 64-bit
@@ -1738,16 +1738,19 @@ int fip_bin_launches(const FipGeom& geo) { return fip_bin_batchable(geo) ? 3 : 4
 // a launch with few items for enough of them to fill the device: two per SM,
 // about 1.4 entries per visibility.  Two, four and eight items per SM wanted,
 // us: three-snapshot calls at 4096^2 929 / 940 / 951 (plain), 568 / 578 / 590
-// (FP16), at 512^2 72 / 76 / 76; chunks of 256 throughout: 943, 590, 76.
+// (FP16), at 512^2 72 / 76 / 76.
 unsigned fip_grid_chunk(size_t nb) {
   const size_t want = (size_t)(1.4 * (double)nb) / (2 * 148);
   return (unsigned)std::max<size_t>(64, std::min<size_t>(FIP_GCHUNK_MAX, want / 32 * 32));
 }
 
 int fip_bin_ctas(int count, size_t nbmax) {
+  // Two CTAs per SM for one snapshot, four for several (eight snapshots of
+  // 0.45 M visibilities: 109 -> 102 us of the three kernels; one of 1.05 M: 43
+  // -> 46).
   const size_t per = (size_t)kBinThreads;
-  return std::max(1, (int)std::min<size_t>(kFipBinCtas / std::max(1, count),
-                                           (nbmax + per - 1) / per));
+  const int most = count > 1 ? kFipBinCtas / count : kFipBinCtas / 2;
+  return std::max(1, (int)std::min<size_t>(most, (nbmax + per - 1) / per));
 }
 
 FipBinSnap fip_bin_snap(const FipGeom& geo, const float* B, int nb, const FipBins& bins,
