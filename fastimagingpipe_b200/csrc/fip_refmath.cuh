@@ -35,29 +35,31 @@ __constant__ float fip_quad_kernel[14] = {
 
 namespace fipref {
 
-// Correctly rounded double quotient x / d for the constant divisors of the
-// chain (180 and pi), by one Markstein correction of the product with the
-// rounded reciprocal: q0 = x * (1/d), e = x - q0 * d (exact with an FMA),
-// q = q0 + e * (1/d) (P. Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  This
-// equals the IEEE division the reference performs (verified against the
-// reference's own targets), at three FP64 operations instead of a division.
-__device__ __forceinline__ double div_const(double x, double d, double rinv) {
-  const double q0 = x * rinv;
-  const double e = fma(-q0, d, x);
-  return fma(e, rinv, q0);
-}
-#define FIP_INV_180 (1.0 / 180.0)
-#define FIP_INV_PI (1.0 / FIP_M_PI)
-// (double)a * M_PI / 180.0, as the reference evaluates the degree-to-radian
-// conversion inside sinf/cosf arguments (FIPkernels.cu:96-97, 116, 135).
+// Correctly rounded products with the constants of the chain's degree
+// conversions.  The reference promotes to double for them, by its double M_PI:
+// (double)a * M_PI / 180.0 inside the arguments of sinf and cosf
+// (FIPkernels.cu:96-97, 116, 135) and (double)(v * 180.0f) / M_PI in the
+// atan2, acos and asin helpers (FIPkernels.cu:145, 157, 169).  Rounded to
+// FP32, both equal fma(v, hi, v * lo) with the constant split into two FP32
+// parts, for every FP32 value of a binade (all 2^23 compared, and with them
+// every v from 2^-90 up, since both forms scale with powers of two; smaller
+// ones would lose v * lo to the flush of denormals, but a mapped pixel's angles
+// are zero or at least 2^-34 degrees).  This is the method of N. Brisebarre and
+// J.-M. Muller, "Correctly rounded multiplication by arbitrary precision
+// constants", IEEE Trans. Comput. 57(2), 2008; the low part of kDegToRad is four
+// ulps above the nearest, which one mantissa of the 2^23 needs.  Two FP32
+// operations stand in for two conversions (a quarter-rate pipe) and three or
+// four FP64 operations.  Explicit intrinsics, so that no contraction of the
+// compiler's can change them.
+constexpr float kDegToRadHi = 0x1.1df46ap-6f;
+constexpr float kDegToRadLo = 0x1.294ea4p-33f;
+constexpr float kRadToDeg180Hi = 0x1.45f306p-2f;
+constexpr float kRadToDeg180Lo = 0x1.b9391p-27f;
 __device__ __forceinline__ float deg_to_rad_arg(float a) {
-  return (float)div_const((double)a * FIP_M_PI, 180.0, FIP_INV_180);
+  return __fmaf_rn(a, kDegToRadHi, __fmul_rn(a, kDegToRadLo));
 }
-// (double)(v * 180.0f) / M_PI, the radian-to-degree step of the reference's
-// atan2/acos/asin helpers (FIPkernels.cu:145, 157, 169).
 __device__ __forceinline__ float rad_to_deg_ret(float v180) {
-  return (float)div_const((double)v180, FIP_M_PI, FIP_INV_PI);
+  return __fmaf_rn(v180, kRadToDeg180Hi, __fmul_rn(v180, kRadToDeg180Lo));
 }
 
 // fmodf(a, 90.0f) == 0, i.e. a is an exact multiple of 90.  fmod is exact,
@@ -65,9 +67,8 @@ __device__ __forceinline__ float rad_to_deg_ret(float v180) {
 // (Sterbenz); only larger angles need the library call.
 __device__ __forceinline__ bool multiple_of_90(float a) {
   const float m = fabsf(a);
-  if (m < 90.0f) return a == 0.0f;
-  if (m < 180.0f) return m == 90.0f;
-  return fmodf(a, 90.0f) == 0;
+  if (m == 0.0f || m == 90.0f) return true;
+  return m >= 180.0f && fmodf(a, 90.0f) == 0;
 }
 
 // computeCeil/computeFloor semantics (FIPkernels.cu:47-61): equal to
@@ -135,13 +136,6 @@ __device__ __forceinline__ float atan2_deg(float y, float x) {
   if (y == 0.0f) return (x >= 0.0f) ? 0.0f : 180.0f;
   if (x == 0.0f) return (y > 0.0f) ? 90.0f : -90.0f;
   return rad_to_deg_ret(atan2f(y, x) * 180.0f);
-}
-
-__device__ __forceinline__ float acos_deg(float v) {
-  if (v >= 1.0f && v - 1.0f < 1e-10) return 0.0f;
-  if (v == 0.0f) return 90.0f;
-  if (v <= -1.0f && v + 1.0f > -1e-10) return 180.0f;
-  return rad_to_deg_ret(acosf(v) * 180.0f);
 }
 
 __device__ __forceinline__ float asin_deg(float v) {
@@ -230,7 +224,9 @@ __device__ __forceinline__ void pixel_target(const Frame& f, int i, int j, int d
   float theta;
   bool mapped = true;
   if (r2 < 0.5f) {
-    theta = acos_deg(sqrtf(r2));
+    // The chain's acos in degrees; its cases at |v| >= 1 are never met here.
+    const float v = sqrtf(r2);
+    theta = v == 0.0f ? 90.0f : rad_to_deg_ret(acosf(v) * 180.0f);
   } else if (r2 <= 1.0f) {
     theta = asin_deg(sqrtf(1.0f - r2));
   } else {
