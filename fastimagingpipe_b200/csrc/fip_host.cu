@@ -1,8 +1,8 @@
 // Host orchestration and C ABI of libfip_b200.so.
 //
 // One fip_imager owns every device buffer of one image size (grid, bins,
-// images, staging), one cuFFT C2R plan and its streams, so repeated calls
-// allocate nothing.  The reference's FIpipe re-allocates ~19 buffers, creates
+// images, staging) and its streams (and, for the sides the transforms here
+// leave out, a cuFFT C2R plan per lane), so repeated calls allocate nothing.  The reference's FIpipe re-allocates ~19 buffers, creates
 // a cuFFT plan and three streams per call and returns 0 whatever happens
 // (FIPkernels.cu:583-861); FIpipe here keeps a small cache of imagers and
 // returns a status.

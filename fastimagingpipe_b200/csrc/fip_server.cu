@@ -26,9 +26,9 @@
 //
 // Beams of image sizes that are not powers of two, or with the scatter
 // reprojection, get an imager of their own and are served one snapshot at a
-// time: the batch engine transforms such sizes with cuFFT, whose plan and
-// work area per step size are made on first use, outside the memory that the
-// group's HBM admission sizes.  Latency is measured per request from submit to
+// time: the batch engine transforms some of these sizes (those with a large
+// prime factor) with cuFFT, whose plan and work area per step size are made on
+// first use, outside the memory that the group's HBM admission sizes.  Latency is measured per request from submit to
 // result.
 #include <cuda_runtime.h>
 
