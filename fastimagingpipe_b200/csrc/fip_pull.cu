@@ -293,7 +293,9 @@ __device__ __forceinline__ float pull_tile(const Plan& p, const float* __restric
     float sum = 0.f;
 #pragma unroll
     for (int e = 0; e < 9; ++e) sum = fmaf(wu[e] * wv[e], q[(e / 3) * kPW + e % 3], sum);
-    const float val = sum * scale;
+    // Sources are magnitudes, so this only turns a NaN (an image whose
+    // visibilities hold an infinity) into 0, as the splat's integer sums do.
+    const float val = fmaxf(sum * scale, 0.f);
     *out = val;
     vmax = fmaxf(vmax, val);
   }

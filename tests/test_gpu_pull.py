@@ -41,3 +41,20 @@ def test_pull_matches_fp64(cuda, n, cell, ha, dec):
             assert relrms(got, want) <= 3e-5
             assert abs(float(mx) - float(img.max())) == 0.0
         im.check()
+
+
+@pytest.mark.parametrize("storage", [fip.STORE_F16, fip.STORE_BF16])
+def test_image_of_nan_pixels_is_zero(cuda, storage):
+    """An infinite visibility leaves NaN in every corrected pixel: the splat's
+    integer sums image those as zero, and so does the pull."""
+    import torch
+    n, cell = 768, 3e-5
+    snap = synthetic.make_snapshots(n_ant=24, radius_m=0.06 / cell, image_size=n, cell_size=cell,
+                                    unit_size=32, n_snap=1, seed=3)
+    d = {k: torch.tensor(getattr(snap, k), device=cuda) for k in ("vis_re", "vis_im", "B", "V")}
+    d["vis_re"][5] = float("inf")
+    img, mx = torch.ones(n, n, device=cuda), torch.ones(1, device=cuda)
+    with fip.Imager(n, snap.num_baselines, cell, 32, form=fip.FORM_PRECISE,
+                    vis_storage=storage) as im:
+        im.image_snapshot(d["vis_re"], d["vis_im"], d["B"], d["V"], snap.num_baselines, img, mx)
+    assert float(img.abs().max()) == 0.0 and float(mx) == 0.0
