@@ -954,7 +954,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_batch(const __grid_constant__
 
 // The reference's pixel mapping for every source pixel: targets[j*N + i] =
 // (LL, MM) of source column i, row j.  Overlapped with the gridding and the FFT
-// on a side stream.  Bound by instruction issue (about 190 a pixel, most of them
+// on a side stream.  Bound by instruction issue (187 a pixel, 239 before, most of them
 // inside atan2f and acosf; 134 MB written at 4096^2, 21 us): FP32 degree
 // conversions in place of FP64 ones took 4096^2 from 124 to 98 us.  Four pixels
 // per thread share the loads of V and the row's terms (two: 101, eight: 103).
