@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_batch(const __grid_constant__
 // inside atan2f and acosf; 134 MB written at 4096^2, 21 us): FP32 degree
 // conversions in place of FP64 ones took 4096^2 from 124 to 97 us (239 to 187
 // instructions a pixel), one test for the special cases and no branch for planes
-// without a tilt to 91.  Four pixels
+// without a tilt to 91 (172).  Four pixels
 // per thread share the loads of V and the row's terms (two: 101, eight: 103).
 constexpr int kTargetsPerThread = 4;
 // ttab: the theta-terms table (fipref::kThetaTabSize entries) or null.
