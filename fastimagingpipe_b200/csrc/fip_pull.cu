@@ -17,9 +17,11 @@
 // Tiles outside the expansion's range (wide cells, odd planes) keep the splat
 // (fip_launch_reproject_gather's rest list).
 //
-// Accuracy: source positions within ~5e-6 pixel of the exact map (FP32
-// rounding of tile-sized offsets, plus the plan's bound on what the expansion
-// leaves out).
+// Accuracy: targets within 1.1e-6 pixel RMS of the exact map over most planes and
+// 1.3e-6 where the coarser form ends (7.5e-6 at most), against the splat's 1.5e-6
+// (9e-6): the FP32 arithmetic of both emulated on the host over 16 geometries.
+// The expansion's origin is the source pixel nearest to the tile centre's source,
+// so that positions round as offsets within a tile.
 //
 // Bound: the FP32 pipes (18 tents, 24 additions, 22 multiply-adds and 13 products
 // a pixel) and shared-memory wavefronts (2.2 a read at a 20 degree turn), both
@@ -27,7 +29,7 @@
 // of plan beside the binning, 3 us for the empty rest list) against 86 us for
 // the splat's 122 instructions a pixel; three-snapshot FP16 calls 632 -> 590
 // us, FP32 674 -> 629; images' error against FP64 unchanged at 4096^2 and 2.3e-6
-// -> 1.0e-6 at 1000^2 (no fixed-point sums).  All-scalar arithmetic: 118
+// -> 1.0e-6 at 1000^2 (no fixed-point sums).  The finer form adds 13 us at 4096^2.  All-scalar arithmetic: 118
 // instructions, 70.5 us.  Five CTAs per SM (48 registers): 71.5 us.  Patch rows
 // of 108 floats: the same.
 #include <cuda_runtime.h>
@@ -56,7 +58,9 @@ struct Plan {
   int a_lo, b_lo;  // patch origin (source pixel; a_lo a multiple of 4)
   int rows;        // patch rows, 0: the tile keeps the splat
   int flags;       // kInner, kFine
-  float ac, bc;    // the centre's source, relative to the patch origin
+  int at;          // patch index of the corner of the 3 x 3 around the origin, the
+                   // source pixel nearest to the tile centre's source
+  float ac, bc;    // the centre's source, relative to the origin (within half a pixel)
   float a00, a01, a10, a11;            // d source / d destination
   float ka, kb, h11, h12, h22;         // second order: source += (ka, kb) quad(dx, dy),
   float lx, ly;                        // third: (ka, kb) quad (lx dx + ly dy)
@@ -65,14 +69,15 @@ struct Plan {
 };
 constexpr int kPlanWords = sizeof(Plan) / 4;
 // kInner: no target of the tile's sources can leave the image.  kFine: the
-// Jacobian is taken at the source rather than at the pixel, and a diagonal
-// step's cross term is kept.
+// nearest source's target is taken to second order in its offset, the Jacobian
+// at the source rather than at the pixel, and a diagonal step's cross term is
+// kept.
 constexpr int kInner = 1, kFine = 2;
 
 // Curvature of the map (pixels per pixel^2) above which a tile is kFine, and
 // above which it keeps the splat; and the bound, in pixels, on the orders left
 // out over the tile (see k_pull_plan).
-constexpr double kCurvFine = 9e-6, kCurvMax = 4.5e-5, kPullSlack = 3e-6;
+constexpr double kCurvFine = 6e-6, kCurvMax = 4.5e-5, kPullSlack = 3e-6;
 
 // kPoly lanes per tile; snapshot blockIdx.y.
 __global__ void __launch_bounds__(kThreads) k_pull_plan(const __grid_constant__ FipGatherBatch in,
@@ -151,9 +156,9 @@ __global__ void __launch_bounds__(kThreads) k_pull_plan(const __grid_constant__ 
     p.lx = (float)(-(N00 * w0 + N10 * w1) / det);
     p.ly = (float)(-(N01 * w0 + N11 * w1) / det);
     // Left out over the tile: the fourth order of the curvature and the slant
-    // term's own third derivative, at the half diagonal; and per source
-    // the curvature over the fraction of a pixel (a quarter of it; three
-    // quarters, and the cross term, without kFine).
+    // term's own third derivative, at the half diagonal; and, without kFine, per
+    // source the curvature over the steps of a pixel or less (three quarters of
+    // it, and the cross term).
     const double wn = fabs(w0) + fabs(w1), curv = wn * is / (s * s * det), R = 46.0;
     const double left = curv * curv * curv * R * R * R * R +
                         0.5 * wn * is * is * sqrt(G0 * G0 + G1 * G1) / (s * s) * R * R * R;
@@ -173,8 +178,10 @@ __global__ void __launch_bounds__(kThreads) k_pull_plan(const __grid_constant__ 
     ok = ok && amax - alo < kPW && bmax - bmin < kPH;
     p.a_lo = alo;
     p.b_lo = bmin;
-    p.ac = (float)(as + (double)(h - alo));
-    p.bc = (float)(bs + (double)(h - bmin));
+    const double ao = rint(as), bo = rint(bs);
+    p.at = ((int)bo + h - bmin - 1) * kPW + (int)ao + h - alo - 1;
+    p.ac = (float)(as - ao);
+    p.bc = (float)(bs - bo);
     p.rows = ok ? bmax - bmin + 1 : 0;
     const bool inner = c0 >= 4 && c0 + kDT + 4 <= 2 * h && r0 >= 4 && r0 + kDT + 4 <= 2 * h;
     p.flags = (inner ? kInner : 0) | (fine ? kFine : 0);
@@ -255,17 +262,20 @@ __device__ __forceinline__ float pull_tile(const Plan& p, const float* __restric
     // of its 3 x 3 (the plan keeps it inside the patch; the bound holds for
     // any plan).
     upk(fma2(src, neg, add2(t, nmagic)), fa, fb);
-    const unsigned idx = (unsigned)((__float_as_int(tb) - kBias) * kPW + (__float_as_int(ta) - kBias) -
-                                    (kPW + 1));
+    const unsigned idx =
+        (unsigned)((__float_as_int(tb) - kBias) * kPW + (__float_as_int(ta) - kBias) + p.at);
     const float* q = patch + min(idx, (unsigned)(kPW * (kPH - 2) - 3));
     f2 ja = fma2(jay, dy2, ja0), jb = fma2(jby, dy2, jb0);
     // Targets of the nearest source and its neighbours relative to the pixel.
     float au, av, bu, bv;
     upk(ja, au, av);
     upk(jb, bu, bv);
-    const float cu = fmaf(fa, au, fb * bu), cv = fmaf(fa, av, fb * bv);
-    const f2 c = pk(cu, cv);
+    float cu = fmaf(fa, au, fb * bu), cv = fmaf(fa, av, fb * bv);
+    f2 c = pk(cu, cv);
     if (FINE) {
+      const float aa = fa * fa, bb = fb * fb, ab = fa * fb;
+      c = fma2(pk(aa, aa), ea, fma2(pk(bb, bb), eb, fma2(pk(ab, ab), eab, c)));
+      upk(c, cu, cv);
       ja = pk(fmaf(p.jx[0], cu, fmaf(p.jy[0], cv, au)), fmaf(p.jx[1], cu, fmaf(p.jy[1], cv, av)));
       jb = pk(fmaf(p.jx[2], cu, fmaf(p.jy[2], cv, bu)), fmaf(p.jx[3], cu, fmaf(p.jy[3], cv, bv)));
     }
