@@ -1688,11 +1688,12 @@ struct fip_batch {
   double phase_ms[kPhases] = {};
   long phase_calls = 0;
   bool phase_pending = false;
-  // Executable graphs of the latest call shapes (snapshots per sequence and
-  // their triggers): a call of a known shape updates its graph in place, so
-  // calls that alternate between shapes, as a server's steps do, do not
-  // instantiate anew (0.3 to 0.5 ms each).  At most kMaxExecs, the least
-  // recently used replaced.
+  // Executable graphs of the latest call shapes -- what decides a call's nodes:
+  // snapshots per sequence, whether a sequence triggers at all (how many triples
+  // changes its launch's extent only), triggers of a slots call -- so a call of a
+  // known shape updates its graph in place, and calls that alternate between
+  // shapes, as a server's steps do, do not instantiate anew (0.3 to 0.5 ms each).
+  // At most kMaxExecs, the least recently used replaced.
   static constexpr size_t kMaxExecs = 8;
   struct Exec {
     std::vector<int> shape;
@@ -2363,15 +2364,15 @@ static int batch_run(fip_batch* b, const int* seq_of, const float* const* vis_re
       FIP_CUDA(cudaGraphKernelNodeSetAttribute(nd, cudaLaunchAttributePriority, &v));
     }
   }
-  // Re-use the executable graph of the call's shape (only pointers, sizes and
-  // launch extents differ); instantiate otherwise.
+  // Re-use the executable graph of the call's shape (only pointers, sizes, launch
+  // extents and the trigger's kernel differ); instantiate otherwise.
   std::vector<int> shape(per, per + nseq);
   if (slots) {
     int triggers = 0;
     for (size_t k = 0; k < count; ++k) triggers += slots[k].prev_image[0] != nullptr;
     shape.push_back(-1 - triggers);
   } else {
-    shape.insert(shape.end(), ntrig, ntrig + nseq);
+    for (int c = 0; c < nseq; ++c) shape.push_back(ntrig[c] > 0);
   }
   fip_batch::Exec* ex = nullptr;
   for (fip_batch::Exec& x : b->execs)
