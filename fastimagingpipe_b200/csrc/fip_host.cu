@@ -122,11 +122,13 @@ class CopyPool {
   void copy(const Seg* segs, int nseg) {
     size_t total = 0;
     for (int k = 0; k < nseg; ++k) total += segs[k].bytes;
-    if (workers_.empty() || total < 2 * kChunk) {
+    // One job at a time: a caller that finds the pool busy copies on its own
+    // thread, beside the other's job, rather than after it.
+    std::unique_lock<std::mutex> call(call_mu_, std::defer_lock);
+    if (workers_.empty() || total < 2 * kChunk || !call.try_lock()) {
       for (int k = 0; k < nseg; ++k) std::memcpy(segs[k].dst, segs[k].src, segs[k].bytes);
       return;
     }
-    std::lock_guard<std::mutex> call(call_mu_);  // one job at a time
     uint32_t n = 0;
     for (int k = 0; k < nseg; ++k)
       for (size_t off = 0; off < segs[k].bytes; off += kChunk) {
