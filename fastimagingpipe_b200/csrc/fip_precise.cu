@@ -38,8 +38,14 @@ constexpr double kLight = 299792458.0;
 // to 1e-300 out of local memory, 99 us, and two serial reductions, 22 us),
 // whose stream-ordered scratch was also mapped anew after every
 // synchronisation (a first pass on a new snapshot: + 0.4 ms).
+// Few rows of many channels are projected by sample, and more than kWarpChans
+// channels summed by every thread (left to one thread per row and one warp, 1 row
+// of 65,536 channels took 2,345 us and 5 rows of 52,500 455; now 29 and 19).
 // ---------------------------------------------------------------------------
 constexpr int kMom = 9;  // sum u' (3), sum u' u'^T (6: 00 01 02 11 12 22), u' = u - uvw[0]
+constexpr int kChan = 2;  // sum k', sum k'^2, k' = k - k of channel 0
+// Channels that one warp sums; more are summed by all threads.
+constexpr size_t kWarpChans = 256;
 
 // Adds the moments of rows first, first + step, ... to acc.
 __device__ __forceinline__ void row_moments(const float* __restrict__ uvw, size_t rows,
@@ -56,18 +62,37 @@ __device__ __forceinline__ void row_moments(const float* __restrict__ uvw, size_
   }
 }
 
-// Sums the CTA's accumulators into out[kMom] (shared memory, ends with a barrier).
-template <int NT>
-__device__ __forceinline__ void block_moments(double (&acc)[kMom], double (*sh)[kMom],
-                                              double* out) {
+// Adds the moments of channels first, first + step, ... to acc.
+__device__ __forceinline__ void channel_moments(const float* __restrict__ freqs, size_t chans,
+                                                size_t first, size_t step, double (&acc)[kChan]) {
+  const double k0 = (double)freqs[0] / kLight;
+  acc[0] = acc[1] = 0.0;
+  for (size_t c = first; c < chans; c += step) {
+    const double d = (double)freqs[c] / kLight - k0;
+    acc[0] += d;
+    acc[1] += d * d;
+  }
+}
+
+// sum k^2 and sum (k - mean k)^2 from the channels' moments.
+__device__ __forceinline__ void channel_sums(const double* mom, const float* __restrict__ freqs,
+                                             size_t chans, double& k2, double& var) {
+  const double k0 = (double)freqs[0] / kLight, n = (double)chans;
+  k2 = n * k0 * k0 + 2.0 * k0 * mom[0] + mom[1];
+  var = fmax(0.0, mom[1] - mom[0] * mom[0] / n);
+}
+
+// Sums the CTA's accumulators into out[K] (shared memory, ends with a barrier).
+template <int NT, int K>
+__device__ __forceinline__ void block_moments(double (&acc)[K], double (*sh)[K], double* out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < kMom; ++k) {
+  for (int k = 0; k < K; ++k) {
     for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
     if (lane == 0) sh[warp][k] = acc[k];
   }
   __syncthreads();
-  if (threadIdx.x < kMom) {
+  if (threadIdx.x < K) {
     double t = 0.0;
 #pragma unroll
     for (int w = 0; w < NT / 32; ++w) t += sh[w][threadIdx.x];
@@ -76,14 +101,14 @@ __device__ __forceinline__ void block_moments(double (&acc)[kMom], double (*sh)[
   __syncthreads();
 }
 
-// The channels' sums by one warp: sum k^2 and sum (k - mean k)^2, mean k.
-__device__ __forceinline__ void channel_sums(const float* __restrict__ freqs, size_t chans,
-                                             double& k2, double& var, double& mean) {
+// The sums of up to kWarpChans channels by one warp: sum k^2 and sum (k - mean k)^2.
+__device__ __forceinline__ void warp_channel_sums(const float* __restrict__ freqs, size_t chans,
+                                                  double& k2, double& var) {
   const int lane = threadIdx.x & 31;
   double s = 0.0;
   for (size_t c = lane; c < chans; c += 32) s += (double)freqs[c] / kLight;
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  mean = s / (double)chans;
+  const double mean = s / (double)chans;
   k2 = 0.0;
   var = 0.0;
   for (size_t c = lane; c < chans; c += 32) {
@@ -225,8 +250,33 @@ __device__ __forceinline__ void project_rows(const float* __restrict__ uvw, size
   }
 }
 
+// The same of samples s0, s0 + step, ... >= skip, one at a time: for few rows.
+__device__ __forceinline__ void project_samples(const float* __restrict__ uvw,
+                                                const float* __restrict__ freqs, size_t rows,
+                                                size_t ns, size_t s0, size_t step,
+                                                const double* b, size_t skip, float* B) {
+  const bool pair = (reinterpret_cast<uintptr_t>(B) & 7) == 0;
+  const double b0 = b[0], b1 = b[1], b2 = b[2], b3 = b[3], b4 = b[4], b5 = b[5];
+  for (size_t s = s0; s < ns; s += step) {
+    if (s < skip) continue;
+    const size_t c = s / rows, r = s - c * rows;
+    const double x = uvw[3 * r], y = uvw[3 * r + 1], z = uvw[3 * r + 2];
+    const double p = x * b0 + y * b1 + z * b2, w = x * b3 + y * b4 + z * b5;
+    const double k = (double)freqs[c] / kLight;
+    if (pair) {
+      reinterpret_cast<float2*>(B)[s] = make_float2((float)(p * k), (float)(w * k));
+    } else {
+      B[2 * s] = (float)(p * k);
+      B[2 * s + 1] = (float)(w * k);
+    }
+  }
+}
+
 constexpr int kPlaneCluster = 8, kPlaneThreads = 1024;
 constexpr int kPlaneChans = 256;  // channels staged at a time
+// Rows below which the projection goes by sample, one cluster's and the spread
+// form's: a quarter of the cluster's threads, one CTA's threads.
+constexpr size_t kFewRowsOne = 2048, kFewRows = kThreads;
 
 // The whole fit in one cluster: moments of an eighth of the rows per CTA,
 // summed through distributed shared memory (the same order in every CTA), the
@@ -237,16 +287,29 @@ __global__ void __cluster_dims__(kPlaneCluster, 1, 1) __launch_bounds__(kPlaneTh
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ double s_warp[kPlaneThreads / 32][kMom];
-  __shared__ double s_mom[kMom], s_all[kMom], s_b[6], s_k[kPlaneChans], s_ch[2];
+  __shared__ double s_chan[kPlaneThreads / 32][kChan];
+  __shared__ double s_mom[kMom], s_all[kMom], s_b[6], s_k[kPlaneChans], s_ch[kChan];
   const size_t first = blockIdx.x * (size_t)kPlaneThreads + threadIdx.x;
   const size_t step = (size_t)kPlaneCluster * kPlaneThreads;
   double acc[kMom];
   row_moments(uvw, rows, first, step, acc);
   block_moments<kPlaneThreads>(acc, s_warp, s_mom);
-  if (threadIdx.x >= kPlaneThreads - 32) {
-    double k2, var, mean;
-    channel_sums(freqs, chans, k2, var, mean);
-    if (threadIdx.x == kPlaneThreads - 1) {
+  if (chans <= kWarpChans) {
+    if (threadIdx.x >= kPlaneThreads - 32) {
+      double k2, var;
+      warp_channel_sums(freqs, chans, k2, var);
+      if (threadIdx.x == kPlaneThreads - 1) {
+        s_ch[0] = k2;
+        s_ch[1] = var;
+      }
+    }
+  } else {  // by every CTA for itself
+    double ch[kChan], k2, var;
+    channel_moments(freqs, chans, threadIdx.x, kPlaneThreads, ch);
+    block_moments<kPlaneThreads>(ch, s_chan, s_ch);
+    channel_sums(s_ch, freqs, chans, k2, var);
+    __syncthreads();
+    if (threadIdx.x == 0) {
       s_ch[0] = k2;
       s_ch[1] = var;
     }
@@ -263,6 +326,11 @@ __global__ void __cluster_dims__(kPlaneCluster, 1, 1) __launch_bounds__(kPlaneTh
     plane_basis(s_all, uvw, rows, chans, s_ch[0], s_ch[1], b);
     for (int k = 0; k < 6; ++k) s_b[k] = b[k];
     if (blockIdx.x == 0) write_basis(b, V);
+  }
+  if (rows < kFewRowsOne && chans > 1) {
+    __syncthreads();
+    project_samples(uvw, freqs, rows, rows * chans, first, step, s_b, 0, B);
+    return;
   }
   for (size_t c0 = 0; c0 < chans; c0 += kPlaneChans) {
     const size_t c1 = c0 + kPlaneChans < chans ? c0 + kPlaneChans : chans;
@@ -282,36 +350,49 @@ __device__ __forceinline__ void put_words(float* p, double v) {
 __device__ __forceinline__ double get_words(const float* p) {
   return __hiloint2double(__float_as_int(p[1]), __float_as_int(p[0]));
 }
-constexpr int kPlaneParts = 148;  // moment CTAs; their sums fill 18 floats of B each
+constexpr int kSums = kMom + kChan;
+constexpr int kPlaneParts = 148;  // moment CTAs; their sums fill 22 floats of B each
 constexpr size_t kPlaneStash = 6;  // samples whose B slots hold the basis until the end
 
 __global__ void __launch_bounds__(kThreads) k_plane_moments(const float* __restrict__ uvw,
-                                                            size_t rows, float* B) {
-  __shared__ double s_warp[kThreads / 32][kMom], s_mom[kMom];
+                                                            const float* __restrict__ freqs,
+                                                            size_t rows, size_t chans, float* B) {
+  __shared__ double s_warp[kThreads / 32][kMom], s_chan[kThreads / 32][kChan], s_mom[kSums];
+  const size_t first = blockIdx.x * (size_t)kThreads + threadIdx.x;
+  const size_t step = (size_t)gridDim.x * kThreads;
   double acc[kMom];
-  row_moments(uvw, rows, blockIdx.x * (size_t)kThreads + threadIdx.x,
-              (size_t)gridDim.x * kThreads, acc);
+  row_moments(uvw, rows, first, step, acc);
   block_moments<kThreads>(acc, s_warp, s_mom);
-  if (threadIdx.x < kMom)
-    put_words(B + 2 * ((size_t)blockIdx.x * kMom + threadIdx.x), s_mom[threadIdx.x]);
+  const bool many = chans > kWarpChans;
+  if (many) {
+    double ch[kChan];
+    channel_moments(freqs, chans, first, step, ch);
+    block_moments<kThreads>(ch, s_chan, s_mom + kMom);
+  }
+  if (threadIdx.x < (many ? kSums : kMom))
+    put_words(B + 2 * ((size_t)blockIdx.x * kSums + threadIdx.x), s_mom[threadIdx.x]);
 }
 
 // One CTA: the partial sums (one moment per warp, ascending within a lane),
 // the basis into V and, as FP64, the head of B.
-__global__ void __launch_bounds__(kMom * 32) k_plane_basis(const float* __restrict__ uvw,
+__global__ void __launch_bounds__(kSums * 32) k_plane_basis(const float* __restrict__ uvw,
                                                            const float* __restrict__ freqs,
                                                            size_t rows, size_t chans, int parts,
                                                            float* B, float* V) {
-  __shared__ double s_mom[kMom];
+  __shared__ double s_mom[kSums];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double t = 0.0;
-  for (int p = lane; p < parts; p += 32) t += get_words(B + 2 * ((size_t)p * kMom + warp));
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (lane == 0) s_mom[warp] = t;
-  double k2 = 0.0, var = 0.0, mean = 0.0;
-  if (warp == 0) channel_sums(freqs, chans, k2, var, mean);
+  const bool many = chans > kWarpChans;
+  if (warp < kMom || many) {
+    double t = 0.0;
+    for (int p = lane; p < parts; p += 32) t += get_words(B + 2 * ((size_t)p * kSums + warp));
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) s_mom[warp] = t;
+  }
+  double k2 = 0.0, var = 0.0;
+  if (warp == 0 && !many) warp_channel_sums(freqs, chans, k2, var);
   __syncthreads();
   if (threadIdx.x == 0) {
+    if (many) channel_sums(s_mom + kMom, freqs, chans, k2, var);
     double b[6];
     plane_basis(s_mom, uvw, rows, chans, k2, var, b);
     for (int k = 0; k < 6; ++k) put_words(B + 2 * k, b[k]);
@@ -320,20 +401,35 @@ __global__ void __launch_bounds__(kMom * 32) k_plane_basis(const float* __restri
 }
 
 // Samples kPlaneStash .. ns - 1: CTA (x, y) takes row blocks x, x + gridDim.x,
-// ... of channels [y per_y, (y + 1) per_y) (at most kPlaneChans).
+// ... of channel blocks y, y + gridDim.y, ... of per_y channels (at most
+// kPlaneChans).
 __global__ void __launch_bounds__(kThreads) k_plane_project(const float* __restrict__ uvw,
                                                             const float* __restrict__ freqs,
                                                             size_t rows, size_t chans,
                                                             size_t per_y, float* B) {
   __shared__ double s_k[kPlaneChans];
-  const size_t c0 = blockIdx.y * per_y, c1 = c0 + per_y < chans ? c0 + per_y : chans;
-  for (size_t c = c0 + threadIdx.x; c < c1; c += kThreads)
-    s_k[c - c0] = (double)freqs[c] / kLight;
   double b[6];
   for (int k = 0; k < 6; ++k) b[k] = get_words(B + 2 * k);
-  __syncthreads();
-  project_rows(uvw, rows, blockIdx.x * (size_t)kThreads + threadIdx.x,
-               (size_t)gridDim.x * kThreads, c0, c1, s_k, b, kPlaneStash, B);
+  for (size_t c0 = blockIdx.y * per_y; c0 < chans; c0 += gridDim.y * per_y) {
+    const size_t c1 = c0 + per_y < chans ? c0 + per_y : chans;
+    for (size_t c = c0 + threadIdx.x; c < c1; c += kThreads)
+      s_k[c - c0] = (double)freqs[c] / kLight;
+    __syncthreads();
+    project_rows(uvw, rows, blockIdx.x * (size_t)kThreads + threadIdx.x,
+                 (size_t)gridDim.x * kThreads, c0, c1, s_k, b, kPlaneStash, B);
+    __syncthreads();
+  }
+}
+
+// The same of fewer than kFewRows rows.
+__global__ void __launch_bounds__(kThreads) k_plane_project_few(const float* __restrict__ uvw,
+                                                                const float* __restrict__ freqs,
+                                                                size_t rows, size_t chans,
+                                                                float* B) {
+  double b[6];
+  for (int k = 0; k < 6; ++k) b[k] = get_words(B + 2 * k);
+  project_samples(uvw, freqs, rows, rows * chans, blockIdx.x * (size_t)kThreads + threadIdx.x,
+                  (size_t)gridDim.x * kThreads, b, kPlaneStash, B);
 }
 
 // The samples whose slots held the basis (one warp).
@@ -449,16 +545,22 @@ cudaError_t fip_launch_plane_project(const float* uvw, const float* freqs, size_
     k_plane_fit<<<kPlaneCluster, kPlaneThreads, 0, s>>>(uvw, freqs, rows, chans, B, V);
     return cudaGetLastError();
   }
-  const int parts = (int)std::min<size_t>(kPlaneParts, (rows + kThreads - 1) / kThreads);
-  k_plane_moments<<<parts, kThreads, 0, s>>>(uvw, rows, B);
-  k_plane_basis<<<1, kMom * 32, 0, s>>>(uvw, freqs, rows, chans, parts, B, V);
+  const size_t most = chans > kWarpChans ? std::max(rows, chans) : rows;
+  const int parts = (int)std::min<size_t>(kPlaneParts, (most + kThreads - 1) / kThreads);
+  k_plane_moments<<<parts, kThreads, 0, s>>>(uvw, freqs, rows, chans, B);
+  k_plane_basis<<<1, kSums * 32, 0, s>>>(uvw, freqs, rows, chans, parts, B, V);
+  if (rows < kFewRows) {
+    const unsigned blocks = (unsigned)std::min<size_t>(8 * 148, (ns + kThreads - 1) / kThreads);
+    k_plane_project_few<<<blocks, kThreads, 0, s>>>(uvw, freqs, rows, chans, B);
+    k_plane_tail<<<1, 32, 0, s>>>(uvw, freqs, rows, B);
+    return cudaGetLastError();
+  }
   // About four CTAs per SM: rows first, channels where the rows are few.
   const size_t bx = std::min<size_t>(4 * 148, (rows + kThreads - 1) / kThreads);
   const size_t want_y = (4 * 148 + bx - 1) / bx;
   size_t per_y = std::max<size_t>(1, (chans + want_y - 1) / want_y);
   per_y = std::min<size_t>(per_y, kPlaneChans);
-  const size_t by = (chans + per_y - 1) / per_y;
-  if (by > 65535) return cudaErrorInvalidValue;
+  const size_t by = std::min<size_t>(65535, (chans + per_y - 1) / per_y);
   k_plane_project<<<dim3((unsigned)bx, (unsigned)by), kThreads, 0, s>>>(uvw, freqs, rows, chans,
                                                                         per_y, B);
   k_plane_tail<<<1, 32, 0, s>>>(uvw, freqs, rows, B);
