@@ -84,11 +84,13 @@ __global__ void k_locate(const float* __restrict__ t, int u, int tile, int n, fl
 // allocation and its release, a memset, a launch and two synchronising
 // copies), 25.2 us in this one (3.9 us of it the kernel; the rest is the wait
 // and the caller); 512 x 512 195 and 163 us.  Beyond that the eight CTAs would
-// become the bound.
+// become the bound.  Two minima are never neighbours, so ceil(u / 2)^2 records
+// always hold them all.
 constexpr int kOneLaunch = 1 << 18, kOneThreads = 1024, kOneCluster = 8;
 struct HostRecords {
   unsigned count;
-  fip_location rec[4095];
+  unsigned cap;  // records the block has room for (host only)
+  __host__ __device__ fip_location* rec() { return reinterpret_cast<fip_location*>(this + 1); }
 };
 __global__ void __cluster_dims__(kOneCluster, 1, 1) __launch_bounds__(kOneThreads)
     k_locate_one(const float* __restrict__ t, int u, int tile, int n, float cell,
@@ -103,14 +105,15 @@ __global__ void __cluster_dims__(kOneCluster, 1, 1) __launch_bounds__(kOneThread
     fip_location L;
     if (!location_at(t, b, u, tile, n, cell, threshold, L)) continue;
     const unsigned k = atomicAdd(count, 1u);
-    if (k < cap) out->rec[k] = L;
+    if (k < cap) out->rec()[k] = L;
   }
   cluster.sync();
   if (blockIdx.x == 0 && threadIdx.x == 0) out->count = s_count;
 }
 
-// Pinned record blocks, one per call in flight (any thread, any device);
-// at most kKeep idle ones are kept, the rest are freed.
+// Pinned record blocks, one per call in flight (any thread, any device), their
+// room a power of two from kLeast records up; at most kKeep idle ones are kept
+// (14.7 MB if all are of the largest size), the rest are freed.
 class RecordPool {
  public:
   static RecordPool& get() {
@@ -118,36 +121,52 @@ class RecordPool {
     static RecordPool& pool = *new RecordPool;
     return pool;
   }
-  HostRecords* take() {
+  // A block with room for `records`: the smallest idle one, or a new one.
+  HostRecords* take(unsigned records) {
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if (!idle_.empty()) {
-        HostRecords* p = idle_.back();
-        idle_.pop_back();
+      auto best = idle_.end();
+      for (auto it = idle_.begin(); it != idle_.end(); ++it)
+        if ((*it)->cap >= records && (best == idle_.end() || (*it)->cap < (*best)->cap)) best = it;
+      if (best != idle_.end()) {
+        HostRecords* p = *best;
+        idle_.erase(best);
         return p;
       }
     }
+    unsigned cap = kLeast;
+    while (cap < records) cap *= 2;
     void* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(HostRecords), cudaHostAllocPortable | cudaHostAllocMapped) !=
-        cudaSuccess) {
+    if (cudaHostAlloc(&p, sizeof(HostRecords) + cap * sizeof(fip_location),
+                      cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
-    return static_cast<HostRecords*>(p);
+    HostRecords* h = static_cast<HostRecords*>(p);
+    h->cap = cap;
+    return h;
   }
+  // Keeps the block; of kKeep + 1 the smallest is freed, so that blocks left by
+  // small matrices do not keep a larger one from staying.
   void give(HostRecords* p) {
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if (idle_.size() < kKeep) {
-        idle_.push_back(p);
-        return;
-      }
+      idle_.push_back(p);
+      if (idle_.size() <= kKeep) return;
+      auto least = std::min_element(idle_.begin(), idle_.end(),
+                                    [](const HostRecords* a, const HostRecords* b) {
+                                      return a->cap < b->cap;
+                                    });
+      p = *least;
+      idle_.erase(least);
     }
     cudaFreeHost(p);
   }
 
  private:
+  RecordPool() { idle_.reserve(kKeep + 1); }
   static constexpr size_t kKeep = 8;
+  static constexpr unsigned kLeast = 4096;
   std::mutex mu_;
   std::vector<HostRecords*> idle_;
 };
@@ -162,7 +181,7 @@ void sort_records(fip_location* rec, size_t count, size_t u) {
 }
 
 // The one-launch form; false when it does not apply (a large matrix, a
-// capturing stream, no pinned memory, more records than a block holds).
+// capturing stream, no pinned memory).
 bool locate_one(const float* tlisi, size_t u, size_t unit_size, size_t image_size,
                 float cell_size, float threshold, fip_location* out, size_t max_out,
                 size_t* found, cudaStream_t s, cudaError_t* err) {
@@ -174,26 +193,24 @@ bool locate_one(const float* tlisi, size_t u, size_t unit_size, size_t image_siz
     return false;
   }
   if (cap != cudaStreamCaptureStatusNone) return false;
-  HostRecords* h = RecordPool::get().take();
+  const unsigned room = (unsigned)((u + 1) / 2 * ((u + 1) / 2));
+  HostRecords* h = RecordPool::get().take(room);
   if (!h) return false;
-  constexpr unsigned kCap = sizeof(h->rec) / sizeof(h->rec[0]);
   k_locate_one<<<kOneCluster, kOneThreads, 0, s>>>(tlisi, (int)u, (int)unit_size, (int)image_size,
-                                         cell_size, threshold, h, kCap);
+                                                   cell_size, threshold, h, h->cap);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     *err = e;  // the block is not reused: the kernel may still write it
     return true;
   }
-  const unsigned count = h->count;
-  const bool fits = count <= kCap;
-  if (fits) {
-    sort_records(h->rec, count, u);
-    for (size_t k = 0; k < count && k < max_out; ++k) out[k] = h->rec[k];
-    *found = count;
-  }
+  const unsigned count = std::min(h->count, h->cap);
+  fip_location* rec = h->rec();
+  sort_records(rec, count, u);
+  for (size_t k = 0; k < count && k < max_out; ++k) out[k] = rec[k];
+  *found = count;
   RecordPool::get().give(h);
-  return fits;
+  return true;
 }
 
 }  // namespace
