@@ -73,8 +73,8 @@ struct Footprint {
 __device__ __forceinline__ bool footprint(float b0, float b1, float scale, int g, Footprint& f) {
   const float hs = (float)(FIP_SUPPORT / 2);
   const int gmin = -(g / 2), gmax = (g - 1) / 2;
-  f.p1 = b0 * scale;
-  f.p2 = b1 * scale;
+  f.p1 = __fmul_rn(b0, scale);
+  f.p2 = __fmul_rn(b1, scale);
   if (!(fabsf(f.p1) < 1e9f && fabsf(f.p2) < 1e9f)) {
     f.a0 = f.b0 = 0;
     f.a1 = f.b1 = -1;
@@ -646,6 +646,12 @@ struct EntryTaps {
   __device__ bool empty() const { return ia_lo >= ia_hi || ib_lo >= ib_hi; }
 };
 
+// EXACT: a tap's distance r - b scale is one rounding of the exact difference, by
+// explicit multiply-adds (precision form); else it is taken from the position
+// rounded to FP32, the order of operations that the plain form keeps
+// (FIPkernels.cu:199-219; half an ulp of hundreds of cells: the grid 1.3e-5 off in
+// relative RMS at 1400^2 with baselines up to the grid's edge, against 5e-7).
+template <bool EXACT>
 __device__ __forceinline__ void entry_taps(const float* __restrict__ B, float scale, int g,
                                            unsigned ent, int trow0, int tcol0, EntryTaps& e) {
   const int v = (int)(ent >> 1), mir = (int)(ent & 1);
@@ -703,20 +709,20 @@ __device__ __forceinline__ void entry_taps(const float* __restrict__ B, float sc
   // r2 = c (direct) or -c (mirrored); on the Nyquist column, always a direct
   // footprint's only one, r2 = -G/2 (r2 never reaches +G/2,
   // FIPkernels.cu:203).  Integers below 2^24: exact in FP32.  The ninth tap
-  // exists only for a position exactly on a cell.  A tap's distance r - b scale is
-  // one rounding of the exact difference, by explicit multiply-adds (from a
-  // position rounded to FP32, half an ulp of hundreds of cells, the grid is 1e-5
-  // off in relative RMS at 1400^2, this way 9e-7).
+  // exists only for a position exactly on a cell.
   const bool down = mir || 2 * c0 == g;
   const float r0 = (float)f.a0, q0 = (float)(down ? -c0 : c0), qs = down ? -1.0f : 1.0f;
+  const auto away = [&](float r, float b, float p) {
+    return EXACT ? __fmaf_rn(-b, scale, r) : __fadd_rn(r, -p);
+  };
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    e.k1[k] = fipref::es(__fmaf_rn(-b0, scale, r0 + (float)k) * ihs);
-    e.k2[k] = fipref::es(__fmaf_rn(-b1, scale, q0 + qs * (float)k) * ihs);
+    e.k1[k] = fipref::es(away(r0 + (float)k, b0, f.p1) * ihs);
+    e.k2[k] = fipref::es(away(q0 + qs * (float)k, b1, f.p2) * ihs);
   }
   e.k1[8] = e.k2[8] = 0.f;
-  if (nr > 8) e.k1[8] = fipref::es(__fmaf_rn(-b0, scale, r0 + 8.0f) * ihs);
-  if (nc > 8) e.k2[8] = fipref::es(__fmaf_rn(-b1, scale, q0 + qs * 8.0f) * ihs);
+  if (nr > 8) e.k1[8] = fipref::es(away(r0 + 8.0f, b0, f.p1) * ihs);
+  if (nc > 8) e.k2[8] = fipref::es(away(q0 + qs * 8.0f, b1, f.p2) * ihs);
 }
 
 // One gridding work item (tile, entry range) of one snapshot, one or two
@@ -743,6 +749,8 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
                                           int4 item, float2* __restrict__ grid,
                                           const FipRawVis& raw = FipRawVis{}) {
   static_assert(FIP_GCHUNK_MAX <= 2 * kThreads, "two entries per thread at most");
+  // The precision form: compensated, or with reduced storage.
+  constexpr bool kExact = COMP || VT == FIP_VIS_F16 || VT == FIP_VIS_BF16;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tile = item.x, cnt = item.z - item.y;
   const int trow0 = (tile / tiles_c) * FIP_GTILE, tcol0 = (tile % tiles_c) * FIP_GTILE;
@@ -798,7 +806,7 @@ __device__ __forceinline__ void grid_item(GridSmem& S, float* s_cre, float* s_ci
 #pragma unroll 1
   for (int left = have ? (more ? 2 : 1) : 0; left > 0; --left, ent = ent2, wr = wr2, wi = wi2) {
     EntryTaps et;
-    entry_taps(B, scale, g, ent, trow0, tcol0, et);
+    entry_taps<kExact>(B, scale, g, ent, trow0, tcol0, et);
     if (et.empty()) continue;
     const float wrf = COMP ? wr : wr * fx, wif = COMP ? wi : wi * fx;
     const int dstep = et.mir ? -kTS : kTS;

@@ -1,4 +1,4 @@
-"""GPU test of the accuracy of the uv grid (both forms, one and two entries per
+"""GPU test of the accuracy of the precision form's uv grid (one and two entries per
 thread) against FP64 sums of the same taps, on baselines over the whole grid.
 
 Tolerance: a tap is the product of two values exp(15.4 (sqrt(1 - x^2) - 1)) in
@@ -17,9 +17,8 @@ import fastimagingpipe_b200 as fip
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("kw", [{}, dict(form=fip.FORM_PRECISE)])
 @pytest.mark.parametrize("n,nb", [(772, 3000), (1024, 1500), (1400, 200000)])
-def test_grid_matches_fp64(cuda, n, nb, kw):
+def test_grid_matches_fp64(cuda, n, nb):
     import torch
     cell = 0.02 / n
     rng = np.random.default_rng(n)
@@ -28,7 +27,7 @@ def test_grid_matches_fp64(cuda, n, nb, kw):
     vis = rng.standard_normal((2, nb)).astype(np.float32)
     V = np.array([0.9, 0.1, 0.4, -0.2, 0.95, 0.2, -0.37, -0.26, 0.88], np.float32)
     d = [torch.tensor(x, device=cuda) for x in (vis[0], vis[1], B.reshape(-1), V)]
-    with fip.Imager(n, nb, cell, 4, **kw) as im:
+    with fip.Imager(n, nb, cell, 4, form=fip.FORM_PRECISE) as im:
         g = im.grid_side
         grid = torch.zeros(g, g // 2 + 1, 2, device=cuda)
         im.grid_snapshot(*d, nb, grid)
