@@ -17,15 +17,21 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kAnyThreads = 256;
-// Run-time lengths: shared memory a CTA may take (sides up to 4,700), and the
-// largest prime factor of M they take.  A prime's pass costs in proportion to
-// it, cuFFT's convolution transform of the whole grid does not; both passes
-// against cuFFT's kernels and the crop, us: p = 199 at 796^2 37 and 44, at 2388^2
-// 208 and 370; p = 251 at 1004^2 53 and 66, p = 211 at 844^2 48 and 45; p =
-// 359 at 1436^2 152 and 120, p = 509 at 2036^2 328 and 225; p = 151 at
-// 3624^2 (whose grid cuFFT splits over several kernels) 551 (before four
-// outputs an item) and 1,069, p = 997 at 3988^2 about 2,250 and 1,512.
-constexpr int kAnySmem = 226 * 1024;
+// Run-time lengths: the largest M (image sides up to 4,800), and the largest
+// prime factor of M they take.  Up to that M two CTAs fit an SM and the passes
+// win whatever the coverage (plain snapshots at 4800^2, baselines up to a fifth,
+// half and nine tenths of the grid's half side: 484, 640 and 952 us, with cuFFT
+// 952, 957 and 983); beyond it one does, and full coverage loses (5000^2 609, 841
+// and 1,346 against 1,116, 1,135 and 1,156; 6000^2 927, 1,293 and 2,030 against
+// 1,417, 1,427 and 1,458).
+// A prime's pass costs in proportion to it, cuFFT's convolution transform of the
+// whole grid does not: the lines are where the passes still win at half of the half
+// side (us, own and cuFFT, at a fifth / half / nine tenths): p = 199 at 1592^2 173,
+// 200, 250 and 239, p = 251 at 2008^2 250, 300, 382 and 325, at 3012^2 490, 644, 840
+// and 880, p = 379 at 3032^2 636, 844, 1,111 and 884, p = 467 at 3736^2 1,034, 1,387,
+// 1,896 and 1,780, p = 509 at 4072^2 1,242, 1,646, 2,211 and 1,765; p = 359 at 1436^2
+// both passes alone 152 against 120.
+constexpr int kAnyMax = 2400;
 constexpr int kAnyPrime = 509;
 static int any_prime_limit(int m) { return m >= 1500 ? kAnyPrime : (m >= 500 ? 251 : 199); }
 
@@ -576,8 +582,7 @@ __global__ void k_correct_c2r(const float* __restrict__ fft_out, const float* __
 static bool plan_any(int g, fipfft::Plan& p) {
   const int m = g / 3;
   p = fipfft::Plan{};
-  if (m < 8 || m % 2 != 0) return false;
-  if (((size_t)fipfft::any_roots(m) + kAnyPrime) * sizeof(float2) > (size_t)kAnySmem) return false;
+  if (m < 8 || m % 2 != 0 || m > kAnyMax) return false;
   int r = m, big[fipfft::kMaxPasses], nbig = 0, e2 = 0, e3 = 0, e5 = 0;
   while (r % 2 == 0) r /= 2, ++e2;
   while (r % 3 == 0) r /= 3, ++e3;

@@ -285,7 +285,7 @@ int fip_imager_set_tuning(fip_imager* im, int fft_values_per_thread, int fft_spl
  * every snapshot with two predecessors (in this call or the previous ones)
  * yields a tLISI matrix (U*U floats, in order, at results); *nresults gets
  * their number.  Asynchronous on `stream`.  Images use the band-pruned
- * transform; sides with a large prime factor, or above 4,700 and no power of
+ * transform; sides with a large prime factor, or above 4,800 and no power of
  * two, one batched cuFFT C2R plan per call size (made before the call's
  * capture, kept for later calls).
  * cfg->reproject must be 0. */

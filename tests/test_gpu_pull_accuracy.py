@@ -45,9 +45,9 @@ def reproject64(pre, V, cell):
     return out.reshape(n, n)
 
 
-def after_grid_error(cuda, n, cell, ha, dec):
+def after_grid_error(cuda, n, cell, ha, dec, border=0):
     """Relative RMS error of one snapshot's image against FP64 steps from its own grid, up to
-    the taper's constant factor."""
+    the taper's constant factor, without `border` pixels along the edges."""
     import torch
     radius = 0.5 / cell * (299792458.0 / 140e6) / 2
     snap = synthetic.make_snapshots(n_ant=60, radius_m=radius, image_size=n, cell_size=cell,
@@ -74,6 +74,8 @@ def after_grid_error(cuda, n, cell, ha, dec):
     t = torch.tensor(t, device=cuda)
     want = reproject64((sky[at][:, at] / (t[:, None] * t[None, :])).abs(), d[3][:9], cell)
     got = img.double()
+    if border:
+        got, want = (x[border:-border, border:-border] for x in (got, want))
     want = want * float((want * got).sum() / (want * want).sum())
     return float((got - want).square().mean().sqrt() / want.square().mean().sqrt())
 
