@@ -86,6 +86,11 @@ __host__ __device__ constexpr size_t fip_qblocks(size_t nb) {
 // image sizes.
 #define FIP_MAX_BATCH 64
 
+// Visibilities of each snapshot of a batched launch.
+struct FipCounts {
+  unsigned nb[FIP_MAX_BATCH];
+};
+
 // One snapshot of a batched gridding launch: its inputs, bins and grid, and
 // its grid geometry (snapshots of a launch may differ in image size).
 struct FipGridSnap {

@@ -730,7 +730,7 @@ static int image_snapshot_impl(fip_imager* im, Lane& L, const float* vr, const f
     if (raw)
       FIP_CUDA(fip_launch_quantize_raw(*raw, nb, vt, L.q_re, L.q_im, L.q_scale, s));
     else
-      FIP_CUDA(fip_launch_quantize(vr, vi, nb, vt, L.q_re, L.q_im, L.q_scale, s));
+      FIP_CUDA(fip_launch_quantize(vr, vi, &nb, vt, L.q_re, L.q_im, L.q_scale, s));
     stage_end(im, k, s);
     im->launches += 1;
     gvr = L.q_re;
@@ -913,7 +913,6 @@ static int image_merged(fip_imager* im, int count, const float* vr, const float*
   int vt = FIP_VIS_F32;
   const bool reduced = precise && im->cfg.vis_storage != FIP_STORE_F32;
   if (reduced) vt = im->cfg.vis_storage == FIP_STORE_F16 ? FIP_VIS_F16 : FIP_VIS_BF16;
-  bool even = true;
   for (int k = 0; k < count; ++k) {
     Lane& K = im->lane[k];
     float* mx = im->maxima + slot0 + k;
@@ -938,21 +937,13 @@ static int image_merged(fip_imager* im, int count, const float* vr, const float*
     gb.nb[k] = (int)nb[k];
     gb.dst[k] = im->images[slot0 + k];
     gb.img_max[k] = reinterpret_cast<unsigned*>(mx);
-    even = even && nb[k] == nb[0];
   }
   // The lanes' list positions together hold ctas * count rows of one launch.
   FIP_CUDA(fip_launch_bin_batch(bin, L.bins.base, s));
-  if (reduced && even) {
-    FIP_CUDA(fip_launch_quantize(vr, vi, nb[0], vt, L.q_re, L.q_im, L.q_scale, s, count,
-                                 vis_stride, im->cfg.max_baselines));
+  if (reduced) {
+    FIP_CUDA(fip_launch_quantize(vr, vi, nb, vt, L.q_re, L.q_im, L.q_scale, s, count, vis_stride,
+                                 im->cfg.max_baselines));
     im->launches += 1;
-  } else if (reduced) {
-    for (int k = 0; k < count; ++k) {
-      Lane& K = im->lane[k];
-      FIP_CUDA(fip_launch_quantize(vr + k * vis_stride, vi + k * vis_stride, nb[k], vt, K.q_re,
-                                   K.q_im, K.q_scale, s));
-      im->launches += 1;
-    }
   }
   FIP_CUDA(fip_launch_grid_batch(in, vt, grid_compensated(precise, vt), s, im->grid_ctas_per_sm));
   FIP_CUDA(fip_launch_fft_cols(geo, L.grid, L.bins.bbox, L.colbuf, im->twiddles, im->fft, s, count,
@@ -1021,7 +1012,7 @@ int fip_grid_snapshot(fip_imager* im, const float* vis_re, const float* vis_im, 
   Lane& L = im->lane[0];
   if (precise && im->cfg.vis_storage != FIP_STORE_F32) {
     vt = im->cfg.vis_storage == FIP_STORE_F16 ? FIP_VIS_F16 : FIP_VIS_BF16;
-    FIP_CUDA(fip_launch_quantize(vis_re, vis_im, nb, vt, L.q_re, L.q_im, L.q_scale, s));
+    FIP_CUDA(fip_launch_quantize(vis_re, vis_im, &nb, vt, L.q_re, L.q_im, L.q_scale, s));
     im->launches += 1;
     gvr = L.q_re;
     gvi = L.q_im;
@@ -1881,7 +1872,7 @@ int batch_record(fip_batch* b, const int* seq_of, const float* const* vr,
     if (reduced) {
       void* qr = static_cast<char*>(q.q_re) + j * q.cfg.max_baselines * 2;
       void* qi = static_cast<char*>(q.q_im) + j * q.cfg.max_baselines * 2;
-      FIP_CUDA(fip_launch_quantize(vr[k], vi[k], nb[k], vt, qr, qi,
+      FIP_CUDA(fip_launch_quantize(vr[k], vi[k], nb + k, vt, qr, qi,
                                    q.q_scale + j * fip_qblocks(q.cfg.max_baselines), bs));
       launches += 1;
     }

@@ -207,9 +207,9 @@ cudaError_t fip_launch_collapse(const float* v0r, const float* v0i, const float*
 // FP16/BF16 storage of a snapshot's visibilities (one launch): scales
 // receives one power-of-two scale per block of FIP_QBLOCK samples
 // ([fip_qblocks(nb)]), out_re/out_im the values divided by their block's.
-// batch > 1: snapshot k's samples at vr + k * in_stride, its results at
-// out + k * out_stride and scales + k * fip_qblocks(out_stride).
-cudaError_t fip_launch_quantize(const float* vr, const float* vi, size_t nb, int vis_type,
+// nb: the counts of the `batch` snapshots; snapshot k's samples at vr + k * in_stride,
+// its results at out + k * out_stride and scales + k * fip_qblocks(out_stride).
+cudaError_t fip_launch_quantize(const float* vr, const float* vi, const size_t* nb, int vis_type,
                                 void* out_re, void* out_im, float* scales, cudaStream_t s,
                                 int batch = 1, size_t in_stride = 0, size_t out_stride = 0);
 // The same from raw two-polarisation samples, collapsed to Stokes I on load.

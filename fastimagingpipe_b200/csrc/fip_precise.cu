@@ -481,11 +481,13 @@ struct RawVis {
 // each): the block's max-abs, its power-of-two scale 2^(e - 14) for a max-abs
 // in [2^e, 2^(e+1)) (so the max lands in [2^14, 2^15), inside FP16's range,
 // and the division by the scale is exact), then the values divided by it.
-// Batched launches: snapshot blockIdx.y.
+// Batched launches: snapshot blockIdx.y, counts.nb[blockIdx.y] samples.
 template <int VT, class L>
-__global__ void __launch_bounds__(kThreads) k_quantize(const L load0, size_t nb, void* qr,
-                                                       void* qi, float* scales,
+__global__ void __launch_bounds__(kThreads) k_quantize(const L load0,
+                                                       const __grid_constant__ FipCounts counts,
+                                                       void* qr, void* qi, float* scales,
                                                        size_t in_stride, size_t out_stride) {
+  const size_t nb = counts.nb[blockIdx.y];
   const L load = load0.at(blockIdx.y * in_stride);
   qr = static_cast<uint16_t*>(qr) + blockIdx.y * out_stride;
   qi = static_cast<uint16_t*>(qi) + blockIdx.y * out_stride;
@@ -493,6 +495,7 @@ __global__ void __launch_bounds__(kThreads) k_quantize(const L load0, size_t nb,
   static_assert(FIP_QBLOCK == 4 * kThreads, "four samples per thread");
   __shared__ float s_max[kThreads / 32];
   const size_t base = (size_t)blockIdx.x * FIP_QBLOCK;
+  if (base >= nb) return;  // a shorter snapshot than the launch's longest
   float re[4], im[4];
   float m = 0.f;
 #pragma unroll
@@ -577,30 +580,35 @@ cudaError_t fip_launch_collapse(const float* v0r, const float* v0i, const float*
 }
 
 template <class L>
-static cudaError_t launch_quantize(const L& load, size_t nb, int vis_type, void* out_re,
+static cudaError_t launch_quantize(const L& load, const size_t* nb, int vis_type, void* out_re,
                                   void* out_im, float* scales, cudaStream_t s, int batch = 1,
                                   size_t in_stride = 0, size_t out_stride = 0) {
-  const size_t blocks = fip_qblocks(nb);
+  if (batch < 1 || batch > FIP_MAX_BATCH) return cudaErrorInvalidValue;
+  FipCounts counts{};
+  size_t blocks = 0;
+  for (int k = 0; k < batch; ++k) {
+    counts.nb[k] = (unsigned)nb[k];
+    if (counts.nb[k] != nb[k]) return cudaErrorInvalidValue;
+    blocks = std::max(blocks, fip_qblocks(nb[k]));
+  }
   if (blocks == 0) return cudaSuccess;
-  if (blocks > 0x7fffffffu) return cudaErrorInvalidValue;
   if (vis_type == FIP_VIS_F16)
     k_quantize<FIP_VIS_F16><<<dim3((unsigned)blocks, batch), kThreads, 0, s>>>(
-        load, nb, out_re, out_im, scales, in_stride, out_stride);
+        load, counts, out_re, out_im, scales, in_stride, out_stride);
   else
     k_quantize<FIP_VIS_BF16><<<dim3((unsigned)blocks, batch), kThreads, 0, s>>>(
-        load, nb, out_re, out_im, scales, in_stride, out_stride);
+        load, counts, out_re, out_im, scales, in_stride, out_stride);
   return cudaGetLastError();
 }
 
-cudaError_t fip_launch_quantize(const float* vr, const float* vi, size_t nb, int vis_type,
+cudaError_t fip_launch_quantize(const float* vr, const float* vi, const size_t* nb, int vis_type,
                                 void* out_re, void* out_im, float* scales, cudaStream_t s,
                                 int batch, size_t in_stride, size_t out_stride) {
-  if (batch < 1 || batch > 65535) return cudaErrorInvalidValue;
   return launch_quantize(F32Vis{vr, vi}, nb, vis_type, out_re, out_im, scales, s, batch,
                          in_stride, out_stride);
 }
 
 cudaError_t fip_launch_quantize_raw(const FipRawVis& raw, size_t nb, int vis_type, void* out_re,
                                     void* out_im, float* scales, cudaStream_t s) {
-  return launch_quantize(RawVis{raw}, nb, vis_type, out_re, out_im, scales, s);
+  return launch_quantize(RawVis{raw}, &nb, vis_type, out_re, out_im, scales, s);
 }
