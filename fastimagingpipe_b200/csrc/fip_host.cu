@@ -424,8 +424,8 @@ static void imager_free(fip_imager* im) {
 }
 
 // The gridder's sums: the precision form's two-limb compensated sums for
-// FP32 (or raw) visibilities; one int32 limb (2^-30 of a work item's summed
-// weights, 2^19 below the rounding of the stored values) for FP16/BF16
+// FP32 (or raw) visibilities; one int32 limb (2^-31 of a work item's summed
+// weights, 2^20 below the rounding of the stored values) for FP16/BF16
 // storage, whose own rounding the compensation could not recover.
 static int grid_compensated(bool precise, int vt) {
   return precise && vt != FIP_VIS_F16 && vt != FIP_VIS_BF16 ? 1 : 0;

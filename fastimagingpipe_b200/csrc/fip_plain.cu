@@ -1755,7 +1755,8 @@ int fip_bin_launches(const FipGeom& geo) { return fip_bin_batchable(geo) ? 3 : 4
 // a launch with few items for enough of them to fill the device: two per SM,
 // about 1.4 entries per visibility.  Two, four and eight items per SM wanted,
 // us: three-snapshot calls at 4096^2 929 / 940 / 951 (plain), 568 / 578 / 590
-// (FP16), at 512^2 72 / 76 / 76.
+// (FP16), at 512^2 72 / 76 / 76.  The 148 is a B200's SMs, fixed so that the
+// bound of the work list (FIP_GITEMS_SPARE) holds whatever the device reports.
 unsigned fip_grid_chunk(size_t nb) {
   const size_t want = (size_t)(1.4 * (double)nb) / (2 * 148);
   return (unsigned)std::max<size_t>(64, std::min<size_t>(FIP_GCHUNK_MAX, want / 32 * 32));

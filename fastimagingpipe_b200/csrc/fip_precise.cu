@@ -16,6 +16,7 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr double kLight = 299792458.0;
+constexpr int kSms = 148;  // of a B200, the one device this is built for
 
 // ---------------------------------------------------------------------------
 // Plane fit of a snapshot's uvw (SVDPreprocessKernels.cu:41-206).  Sample
@@ -351,7 +352,7 @@ __device__ __forceinline__ double get_words(const float* p) {
   return __hiloint2double(__float_as_int(p[1]), __float_as_int(p[0]));
 }
 constexpr int kSums = kMom + kChan;
-constexpr int kPlaneParts = 148;  // moment CTAs; their sums fill 22 floats of B each
+constexpr int kPlaneParts = kSms;  // moment CTAs; their sums fill 22 floats of B each
 constexpr size_t kPlaneStash = 6;  // samples whose B slots hold the basis until the end
 
 __global__ void __launch_bounds__(kThreads) k_plane_moments(const float* __restrict__ uvw,
@@ -553,14 +554,14 @@ cudaError_t fip_launch_plane_project(const float* uvw, const float* freqs, size_
   k_plane_moments<<<parts, kThreads, 0, s>>>(uvw, freqs, rows, chans, B);
   k_plane_basis<<<1, kSums * 32, 0, s>>>(uvw, freqs, rows, chans, parts, B, V);
   if (rows < kFewRows) {
-    const unsigned blocks = (unsigned)std::min<size_t>(8 * 148, (ns + kThreads - 1) / kThreads);
+    const unsigned blocks = (unsigned)std::min<size_t>(8 * kSms, (ns + kThreads - 1) / kThreads);
     k_plane_project_few<<<blocks, kThreads, 0, s>>>(uvw, freqs, rows, chans, B);
     k_plane_tail<<<1, 32, 0, s>>>(uvw, freqs, rows, B);
     return cudaGetLastError();
   }
   // About four CTAs per SM: rows first, channels where the rows are few.
-  const size_t bx = std::min<size_t>(4 * 148, (rows + kThreads - 1) / kThreads);
-  const size_t want_y = (4 * 148 + bx - 1) / bx;
+  const size_t bx = std::min<size_t>(4 * kSms, (rows + kThreads - 1) / kThreads);
+  const size_t want_y = (4 * kSms + bx - 1) / bx;
   size_t per_y = std::max<size_t>(1, (chans + want_y - 1) / want_y);
   per_y = std::min<size_t>(per_y, kPlaneChans);
   const size_t by = std::min<size_t>(65535, (chans + per_y - 1) / per_y);
@@ -574,7 +575,7 @@ cudaError_t fip_launch_collapse(const float* v0r, const float* v0i, const float*
                                 const float* v3i, const unsigned char* f0,
                                 const unsigned char* f3, const float* w0, const float* w3,
                                 float* out_re, float* out_im, size_t ns, cudaStream_t s) {
-  const int blocks = (int)std::min<size_t>(4 * 148, (ns + kThreads - 1) / kThreads + 1);
+  const int blocks = (int)std::min<size_t>(4 * kSms, (ns + kThreads - 1) / kThreads + 1);
   k_collapse<<<blocks, kThreads, 0, s>>>(v0r, v0i, v3r, v3i, f0, f3, w0, w3, out_re, out_im, ns);
   return cudaGetLastError();
 }

@@ -23,15 +23,15 @@
 // The expansion's origin is the source pixel nearest to the tile centre's source,
 // so that positions round as offsets within a tile.
 //
-// Bound: the FP32 pipes (18 tents, 24 additions, 22 multiply-adds and 13 products
-// a pixel) and shared-memory wavefronts (2.2 a read at a 20 degree turn), both
-// near 75 %; 101 instructions a pixel at 73 % issue.  4096^2: 68 us (and 6 us
-// of plan beside the binning, 3 us for the empty rest list) against 86 us for
-// the splat's 122 instructions a pixel; three-snapshot FP16 calls 632 -> 590
-// us, FP32 674 -> 629; images' error against FP64 unchanged at 4096^2 and 2.3e-6
-// -> 1.0e-6 at 1000^2 (no fixed-point sums).  The finer form adds 13 us at 4096^2.  All-scalar arithmetic: 118
-// instructions, 70.5 us.  Five CTAs per SM (48 registers): 71.5 us.  Patch rows
-// of 108 floats: the same.
+// Bound: instruction issue (18 tents, 24 additions, 22 multiply-adds and 13
+// products among 102 instructions a pixel, 74 % of the issue slots) with the
+// shared-memory loads (2.3 wavefronts a read at a 20 degree turn, 64 % of their
+// rate) beside it.  4096^2: 68 us (and 6 us of plan beside the binning, 3 us for
+// the empty rest list) against 86 us for the splat's 122 instructions a pixel;
+// three-snapshot FP16 calls 632 -> 590 us, FP32 674 -> 629; images' error against
+// FP64 2.3e-6 -> 1.2e-6 at 1024^2 (no fixed-point sums).  The finer form of curved
+// tiles adds 13 us.  All-scalar arithmetic: 118 instructions, 70.5 us.  Five CTAs
+// per SM (48 registers): 71.5 us.  Patch rows of 108 floats: the same.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

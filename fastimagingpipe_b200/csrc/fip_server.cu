@@ -26,10 +26,11 @@
 //
 // Beams of image sizes that are not powers of two, or with the scatter
 // reprojection, get an imager of their own and are served one snapshot at a
-// time: the batch engine transforms some of these sizes (those with a large
-// prime factor) with cuFFT, whose plan and work area per step size are made on
-// first use, outside the memory that the group's HBM admission sizes.  Latency is measured per request from submit to
-// result.
+// time.  Only sides without a transform of the library's own need that (the
+// batch engine images them with cuFFT, whose plan and work area per step size
+// are made on first use, outside the memory that the group's HBM admission
+// sizes); the line at powers of two (batchable) takes in more.  Latency is
+// measured per request from submit to result.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -95,7 +96,9 @@ struct Group {
   // submit writes a request's inputs where the step's upload reads them, one
   // copy by several threads (40 us for 130,816 visibilities) instead of two by
   // one (130 to 370 us in submit alone).  A request that finds none free takes
-  // vectors.
+  // vectors.  The copying threads are the host-buffer calls' pool
+  // (fip_host_copy): a submit that finds it busy copies by itself, and its three
+  // threads poll for 2 ms after a submit of half a megabyte or more.
   std::vector<float*> idle_inputs;
   size_t stride() const { return 4 * nb + 16; }
 };

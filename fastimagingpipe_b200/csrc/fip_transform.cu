@@ -479,10 +479,12 @@ __global__ void __launch_bounds__(split_threads<LM, LE>(), (LE == 4 ? 6 : 4))
 // The two passes for run-time lengths (fip_fft_any.cuh): a CTA per column or row
 // pair in turn, several CTAs per SM hiding one another's barriers; inputs,
 // outputs and epilogue as the power-of-two passes'.  Bound: shared-memory
-// round trips and barriers.  Both passes against cuFFT's transform of the whole
-// grid and the crop, us: 1000^2 15 and 39, 1500^2 24 and 55, 3000^2 80 and 230,
-// 1484^2 (factor 53) 60 and 120; the band layout they allow also spares the
-// gridder the rest of the grid (3000^2 66 -> 45 us).
+// round trips and barriers (44 % of issue slots, three CTAs per SM at 3000^2).
+// Both passes against cuFFT's transform of the whole grid and the crop, us:
+// 1000^2 15 and 39, 1500^2 24 and 55, 1484^2 (factor 53) 60 and 120, 3000^2 93 and
+// 236 with baselines up to three tenths of the grid's half side, 198 and 237 up to
+// nine tenths; the band layout they allow also spares the gridder the rest of the
+// grid (3000^2 66 -> 45 us).
 __global__ void __launch_bounds__(kAnyThreads) k_fft_any_cols(const float2* __restrict__ H,
                                                               const unsigned* __restrict__ bbox,
                                                               float2* __restrict__ P,

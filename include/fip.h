@@ -144,7 +144,9 @@ int fip_image_snapshot_raw(fip_imager* im, const fip_raw_vis* raw, const float* 
  * (interleaved float pairs, row-major, G = ceil(1.5 N)), holding
  * h(r1, r2) = (g(r1, r2) + conj g(-r1, -r2)) / 2 at row r1 mod G, column
  * r2 >= 0, where g is the reference's grid without its (-1)^(r1+r2)
- * checkerboard.  This is the input layout of a C2R transform.
+ * checkerboard.  This is the input layout of a C2R transform.  A visibility's
+ * position b * cell * G is rounded to FP32 before its taps in the plain form (up
+ * to 3e-5 cell at the edge of a 1000-cell grid), and is not in the precision form.
  */
 int fip_grid_snapshot(fip_imager* im, const float* vis_re, const float* vis_im, const float* B,
                       const float* V, size_t nb, float* grid, void* stream);
